@@ -103,6 +103,7 @@ hp::SolveConsts consts_of(const hp_params* p) {
     if (p->precision == HP_PRECISION_F16ACC && p->debug_checked_taps) sc.soft_mask |= hp::SOFT_MASK_CHECKED;
     sc.tile_h = p->tile_h > 0 ? p->tile_h : hp::TILE_H;
     sc.staging = p->staging > 0 ? p->staging : 4;
+    sc.memo = 1;
     return sc;
 }
 
@@ -358,7 +359,8 @@ hp::BatchList batch_of(const Prepared& P, int list) {
 }
 
 // Copy a job's packed state out to the caller's maps.
-hp_status export_maps(hp_ctx* ctx, const Prepared& P, int k, hp_maps* m, bool want_depth_normal, bool want_cost) {
+hp_status export_maps(hp_ctx* ctx, const Prepared& P, int k, hp_maps* m, bool want_depth_normal, bool want_cost,
+                      bool raw_cost = false) {
     const hp::ViewDesc& v = P.host[k];
     const size_t px = static_cast<size_t>(v.W) * v.H;
     float* d = want_depth_normal ? m->depth : nullptr;
@@ -367,7 +369,7 @@ hp_status export_maps(hp_ctx* ctx, const Prepared& P, int k, hp_maps* m, bool wa
     float* cf = want_cost ? m->confidence : nullptr;
     if (m->memory == HP_MEMORY_DEVICE) {
         HP_CUDA(counted(ctx, HP_KERNEL_OTHER,
-                        [&] { return hp::launch_unpack(P.host.data(), k, d, nrm, c, cf, ctx->stream); }));
+                        [&] { return hp::launch_unpack(P.host.data(), k, d, nrm, c, cf, ctx->stream, raw_cost); }));
         return HP_OK;
     }
     HP_CUDA(ctx->staging.ensure(px * 6 * sizeof(float)));
@@ -377,7 +379,7 @@ hp_status export_maps(hp_ctx* ctx, const Prepared& P, int k, hp_maps* m, bool wa
     float* scf = sc + px;
     HP_CUDA(counted(ctx, HP_KERNEL_OTHER, [&] {
         return hp::launch_unpack(P.host.data(), k, d ? sd : nullptr, nrm ? sn : nullptr, c ? sc : nullptr,
-                                 cf ? scf : nullptr, ctx->stream);
+                                 cf ? scf : nullptr, ctx->stream, raw_cost);
     }));
     if (d) HP_CUDA(cudaMemcpyAsync(d, sd, px * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
     if (nrm) HP_CUDA(cudaMemcpyAsync(nrm, sn, 3 * px * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream));
@@ -424,8 +426,9 @@ hp_status launch_cost(hp_ctx* ctx, const hp::BatchList& bl, const hp_params* p) 
     return HP_OK;
 }
 
-hp_status launch_pass(hp_ctx* ctx, const hp::BatchList& bl, const hp_params* p, int it, int color) {
+hp_status launch_pass(hp_ctx* ctx, const hp::BatchList& bl, const hp_params* p, int it, int color, bool memo = true) {
     hp::SolveConsts sc = consts_of(p);
+    sc.memo = memo;
     cudaError_t e = counted(ctx, HP_KERNEL_PROPAGATE, [&] {
         return p->precision == HP_PRECISION_F16ACC ? hp::launch_propagate_f16(bl, sc, it, color, ctx->stream)
                                                    : hp::launch_propagate_f32(bl, sc, it, color, ctx->stream);
@@ -822,8 +825,8 @@ hp_status hp_propagate_pass(hp_ctx* ctx, const hp_job* job, const hp_params* par
     Prepared P;
     if ((st = prepare(ctx, job, 1, params, &P)) != HP_OK) return st;
     if ((st = import_maps(ctx, P, 0, maps, true)) != HP_OK) return st;
-    if ((st = launch_pass(ctx, batch_of(P, 0), params, iteration, color)) != HP_OK) return st;
-    if ((st = export_maps(ctx, P, 0, maps, true, true)) != HP_OK) return st;
+    if ((st = launch_pass(ctx, batch_of(P, 0), params, iteration, color, false)) != HP_OK) return st;
+    if ((st = export_maps(ctx, P, 0, maps, true, true, true)) != HP_OK) return st;
     HP_CUDA(cudaStreamSynchronize(ctx->stream));
     flush_profile(ctx);
     return HP_OK;

@@ -567,11 +567,6 @@ __device__ __forceinline__ float cost_f16(RefStats st, const __half2* s_win, con
     return __fdiv_rn(sum, static_cast<float>(kk));
 }
 
-__device__ __forceinline__ bool same_plane16(float4 a, float4 b) {
-    return __float_as_uint(a.x) == __float_as_uint(b.x) && __float_as_uint(a.y) == __float_as_uint(b.y) &&
-           __float_as_uint(a.z) == __float_as_uint(b.z) && __float_as_uint(a.w) == __float_as_uint(b.w);
-}
-
 template <int R, int ST, int TH, int D>
 __device__ __forceinline__ void tile_cost16(const ViewDesc* v, int tile_x, int tile_y, const SolveConsts& sc,
                                             float* s_ref, __half2* s_win) {
@@ -643,27 +638,12 @@ __device__ __forceinline__ void tile_propagate16(const ViewDesc* v, int tile_x, 
     float4 best = make_float4(0.f, 0.f, 0.f, 0.f);
     float best_cost = 0.f;
     unsigned need = 0;
+    bool settled = true;
     if (active) {
         st = load_window<R, ST, NT>(s_win, s_ref, tw, lx, ly);
         best = v->hyp[idx];
-        best_cost = v->cost[idx];
-#pragma unroll
-        for (int cand = 0; cand < 4; ++cand) {
-            const int nxp = x + (cand == 0 ? -1 : (cand == 1 ? 1 : 0));
-            const int nyp = y + (cand == 2 ? -1 : (cand == 3 ? 1 : 0));
-            if (nxp < 0 || nxp >= W || nyp < 0 || nyp >= H) continue;
-            const float4 h = v->hyp[static_cast<size_t>(nyp) * W + nxp];
-            if (h.x < dmin || h.x > dmax) continue;
-            bool dup = same_plane16(h, best);
-            for (int j = 0; j < cand && !dup; ++j) {
-                if (need & (1u << j)) {
-                    const int jx = x + (j == 0 ? -1 : (j == 1 ? 1 : 0));
-                    const int jy = y + (j == 2 ? -1 : (j == 3 ? 1 : 0));
-                    dup = same_plane16(h, v->hyp[static_cast<size_t>(jy) * W + jx]);
-                }
-            }
-            if (!dup) need |= 1u << cand;
-        }
+        best_cost = cost_value(v->cost[idx]);
+        need = neighbour_needs(v, x, y, best, sc.memo && iteration > 0);
     }
     sm.stat[threadIdx.x] = make_float2(st.mean, st.ssd);
     const int cnt = __popc(need);
@@ -716,6 +696,7 @@ __device__ __forceinline__ void tile_propagate16(const ViewDesc* v, int tile_x, 
                 const int nxp = x + (cand == 0 ? -1 : (cand == 1 ? 1 : 0));
                 const int nyp = y + (cand == 2 ? -1 : (cand == 3 ? 1 : 0));
                 best_cost = c;
+                settled = false;
                 best = v->hyp[static_cast<size_t>(nyp) * W + nxp];
             }
         }
@@ -742,13 +723,14 @@ __device__ __forceinline__ void tile_propagate16(const ViewDesc* v, int tile_x, 
                                         sc.top_k, sc.soft_mask);
         if (c < best_cost) {
             best_cost = c;
+            settled = false;
             best = make_float4(cd, cn.x, cn.y, cn.z);
         }
         drange = __fmul_rn(drange, sc.step_decay);
         nrange = __fmul_rn(nrange, sc.step_decay);
     }
     v->hyp[idx] = best;
-    v->cost[idx] = best_cost;
+    v->cost[idx] = sc.memo && settled ? -best_cost : best_cost;
 }
 
 template <int R, int ST, int TH, int D>

@@ -13,7 +13,7 @@
 // external-maps kernel give the same bits on the same inputs.
 #pragma once
 
-#include "hp_internal.h"
+#include "hp_tile.cuh"
 
 namespace hp {
 
@@ -66,7 +66,7 @@ __device__ __forceinline__ void tile_filter(const ViewDesc* __restrict__ views, 
         if (x >= W) continue;
         const size_t i = static_cast<size_t>(y) * W + x;
         float4 h = __ldcg(v->hyp + i);
-        float c = __ldcg(v->cost + i);
+        float c = cost_value(__ldcg(v->cost + i));
         const bool keep = h.x > 0.0f && filter_agreeing(f, W, H, x, y, h.x, h.y, h.z, h.w, fetch) >= f->min_consistent;
         if (!keep) {
             if (h.x > 0.0f) {

@@ -32,7 +32,7 @@ struct ViewDesc {
     float kinv[9];
     alignas(16) float ab[HP_MAX_SOURCES][12];  // A (9), b (3) per source; 16-byte aligned rows
     float4* hyp;                      // H*W
-    float* cost;                      // H*W
+    float* cost;                      // H*W; sign bit: see cost_settled (hp_tile.cuh)
     int ref_pitch, ref16_pitch;
     int W, H, S;
     int tiles_x, tiles_y;
@@ -67,6 +67,7 @@ struct SolveConsts {
     unsigned soft_mask;  // FP16 path: sources sampled in software (bit per source); SOFT_MASK_CHECKED
     int tile_h;          // rows of a CTA's tile (TILE_W x tile_h pixels, tile_h warps): 8, or 4 (FP16 path)
     int staging;         // FP16 path: quad loads in flight per window row, 4 or 8
+    int memo;            // half-passes keep and use the settled bit of stored costs (whole solves: 1)
 };
 
 // A batch launch covers the tiles of several views: view k owns flattened
@@ -208,8 +209,9 @@ cudaError_t launch_quads(const __half* src16, int pitch16, int W, int H, uint2* 
 // (2 radius + 1)^2 square covers it, -1 for none.
 cudaError_t launch_seed_map(const hp_seed* seeds, int num_seeds, int radius, int W, int H, int* map,
                             cudaStream_t st);
+// raw_cost: costs as stored (a caller's own, any sign); else without the settled bit.
 cudaError_t launch_unpack(const ViewDesc* views_host_copy, int view, float* depth, float* normal, float* cost,
-                          float* conf, cudaStream_t st);
+                          float* conf, cudaStream_t st, bool raw_cost = false);
 cudaError_t launch_pack(const ViewDesc* views_host_copy, int view, const float* depth, const float* normal,
                         const float* cost, cudaStream_t st);
 // The filter stage of view `view` (views: device descriptors; tiles: its tile

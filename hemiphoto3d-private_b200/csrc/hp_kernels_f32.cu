@@ -237,11 +237,6 @@ __device__ __forceinline__ float cost_f32(const float* __restrict__ s_ref, int t
     return sum / static_cast<float>(k);
 }
 
-__device__ __forceinline__ bool same_plane(float4 a, float4 b) {
-    return __float_as_uint(a.x) == __float_as_uint(b.x) && __float_as_uint(a.y) == __float_as_uint(b.y) &&
-           __float_as_uint(a.z) == __float_as_uint(b.z) && __float_as_uint(a.w) == __float_as_uint(b.w);
-}
-
 __global__ void __launch_bounds__(256) init_kernel(BatchList bl) {
     int tile_x, tile_y;
     const ViewDesc* v = locate_tile(bl, blockIdx.x, &tile_x, &tile_y);
@@ -323,26 +318,11 @@ __device__ __forceinline__ void tile_propagate(const ViewDesc* v, int tile_x, in
     float4 best = make_float4(0.f, 0.f, 0.f, 0.f);
     float best_cost = 0.f;
     unsigned need = 0;
+    bool settled = true;
     if (active) {
         best = v->hyp[idx];
-        best_cost = v->cost[idx];
-#pragma unroll
-        for (int cand = 0; cand < 4; ++cand) {
-            const int nxp = x + (cand == 0 ? -1 : (cand == 1 ? 1 : 0));
-            const int nyp = y + (cand == 2 ? -1 : (cand == 3 ? 1 : 0));
-            if (nxp < 0 || nxp >= W || nyp < 0 || nyp >= H) continue;
-            const float4 h = v->hyp[static_cast<size_t>(nyp) * W + nxp];
-            if (h.x < dmin || h.x > dmax) continue;
-            bool dup = same_plane(h, best);
-            for (int j = 0; j < cand && !dup; ++j) {
-                if (need & (1u << j)) {
-                    const int jx = x + (j == 0 ? -1 : (j == 1 ? 1 : 0));
-                    const int jy = y + (j == 2 ? -1 : (j == 3 ? 1 : 0));
-                    dup = same_plane(h, v->hyp[static_cast<size_t>(jy) * W + jx]);
-                }
-            }
-            if (!dup) need |= 1u << cand;
-        }
+        best_cost = cost_value(v->cost[idx]);
+        need = neighbour_needs(v, x, y, best, sc.memo && iteration > 0);
     }
     // Exclusive scan of the item counts over the warp, then over the CTA's warps; owners write their items.
     const int cnt = __popc(need);
@@ -389,6 +369,7 @@ __device__ __forceinline__ void tile_propagate(const ViewDesc* v, int tile_x, in
                 const int nxp = x + (cand == 0 ? -1 : (cand == 1 ? 1 : 0));
                 const int nyp = y + (cand == 2 ? -1 : (cand == 3 ? 1 : 0));
                 best_cost = c;
+                settled = false;
                 best = v->hyp[static_cast<size_t>(nyp) * W + nxp];
             }
         }
@@ -416,13 +397,14 @@ __device__ __forceinline__ void tile_propagate(const ViewDesc* v, int tile_x, in
         const float c = cost_f32<R, ST>(s_ref, tw, lx, ly, x, y, cd, cn.x, cn.y, cn.z, v, sc.top_k);
         if (c < best_cost) {
             best_cost = c;
+            settled = false;
             best = make_float4(cd, cn.x, cn.y, cn.z);
         }
         drange = __fmul_rn(drange, sc.step_decay);
         nrange = __fmul_rn(nrange, sc.step_decay);
     }
     v->hyp[idx] = best;
-    v->cost[idx] = best_cost;
+    v->cost[idx] = sc.memo && settled ? -best_cost : best_cost;
 }
 
 template <int R, int ST>

@@ -46,6 +46,62 @@ __device__ __forceinline__ void tile_init(const ViewDesc* v, int tile_x, int til
     }
 }
 
+// Stored costs carry one bit of history.  A cost is never negative, so the sign
+// bit of v->cost marks a pixel whose last half-pass left its plane as it was
+// ("settled"); readers of the cost itself drop it with cost_value.
+__device__ __forceinline__ float cost_value(float c) { return fabsf(c); }
+__device__ __forceinline__ bool cost_settled(float c) { return (__float_as_uint(c) >> 31) != 0u; }
+
+__device__ __forceinline__ bool same_plane(float4 a, float4 b) {
+    return __float_as_uint(a.x) == __float_as_uint(b.x) && __float_as_uint(a.y) == __float_as_uint(b.y) &&
+           __float_as_uint(a.z) == __float_as_uint(b.z) && __float_as_uint(a.w) == __float_as_uint(b.w);
+}
+
+// The neighbour planes (bit 0..3: left, right, up, down) that pixel (x, y) must
+// score in this half-pass.  Left out, because none of them can win:
+//  - a plane outside the depth range (the reference's rule);
+//  - a plane bit-identical to the pixel's own or to an earlier listed one:
+//    same pixel, same plane, same arithmetic, same cost;
+//  - with `memo`, the plane of a settled neighbour, and any plane identical to
+//    one.  The neighbour is of the other color, so exactly one half-pass of its
+//    own lies between two visits of this pixel: a settled neighbour holds the
+//    plane it held at this pixel's previous visit, which scored it then (or a
+//    bit-identical one).  The pixel's cost has been at most that score ever
+//    since, and a candidate must be strictly lower.  `memo` is false where no
+//    previous visit by the same solve exists: in iteration 0, and in a single
+//    half-pass on caller maps.
+// On 1920 x 1080, r 7, s 2, 6 sources, 12 iterations this leaves 1.54 of the
+// 1.78 planes per visit the identity rule alone leaves (3000 x 2000 with noise,
+// 8 sources: 1.53 of 1.94).
+__device__ __forceinline__ unsigned neighbour_needs(const ViewDesc* v, int x, int y, float4 own, bool memo) {
+    const int W = v->W, H = v->H;
+    const float dmin = v->dmin, dmax = v->dmax;
+    unsigned need = 0, settled = 0;
+    auto at = [&](int cand) {
+        return static_cast<size_t>(y + (cand == 2 ? -1 : (cand == 3 ? 1 : 0))) * W + x +
+               (cand == 0 ? -1 : (cand == 1 ? 1 : 0));
+    };
+#pragma unroll
+    for (int cand = 0; cand < 4; ++cand) {
+        const bool inside = cand == 0 ? x > 0 : (cand == 1 ? x + 1 < W : (cand == 2 ? y > 0 : y + 1 < H));
+        if (inside) {
+            need |= 1u << cand;
+            if (memo && cost_settled(v->cost[at(cand)])) settled |= 1u << cand;
+        }
+    }
+    need &= ~settled;
+#pragma unroll
+    for (int cand = 0; cand < 4; ++cand) {
+        if (!(need & (1u << cand))) continue;
+        const float4 h = v->hyp[at(cand)];
+        bool drop = h.x < dmin || h.x > dmax || same_plane(h, own);
+        for (int j = 0; j < 4 && !drop; ++j)
+            if (((j < cand ? need : 0u) | settled) & (1u << j)) drop = same_plane(h, v->hyp[at(j)]);
+        if (drop) need &= ~(1u << cand);
+    }
+    return need;
+}
+
 // Final stage of a view in a persistent launch: its tile's packed state into
 // the output maps (depth, camera-frame AoS normal, cost, and confidence
 // 1 - cost / 2 when wanted).
@@ -65,7 +121,7 @@ __device__ __forceinline__ void tile_unpack(const ViewDesc* v, int tile_x, int t
         v->out_normal[3 * i] = h.y;
         v->out_normal[3 * i + 1] = h.z;
         v->out_normal[3 * i + 2] = h.w;
-        const float c = __ldcg(v->cost + i);
+        const float c = cost_value(__ldcg(v->cost + i));
         v->out_cost[i] = c;
         if (v->out_conf) v->out_conf[i] = __fsub_rn(1.0f, __fmul_rn(c, 0.5f));
     }
