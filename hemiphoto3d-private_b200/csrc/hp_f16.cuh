@@ -94,7 +94,6 @@ template <int V> struct WinRow;
 template <> struct WinRow<1> { using T = unsigned; };
 template <> struct WinRow<2> { using T = uint2; };
 template <> struct WinRow<4> { using T = uint4; };
-constexpr int WIN_PAIRS_MAX = 32;
 
 // Per-pixel window statistics; the mean-subtracted window itself goes to s_win,
 // laid out [row][thread][VEC half2]: one row of a pixel's residual pairs is one
@@ -103,6 +102,27 @@ constexpr int WIN_PAIRS_MAX = 32;
 struct RefStats {
     float mean;  // window mean (the shift of every sum)
     float ssd;   // sum (r - mean)^2
+};
+
+// Shared memory of a CTA (dynamic: the widest windows pass the 48 KB static
+// limit).  Windows kept in s_win need the reference tile only while they are
+// built, so the half-pass's source costs then take its place.
+template <int R, int ST, int TH>
+struct alignas(16) Shared {
+    static constexpr int NT = 32 * TH;
+    static constexpr int REF = (TILE_W + 2 * R) * (TH + 2 * R);
+    static constexpr int UNITS = HP_MAX_SOURCES * NT;
+    static constexpr bool OVERLAY = Win<R, ST>::IN_SMEM;
+    __half2 win[OVERLAY ? Win<R, ST>::SIDE * Win<R, ST>::VEC * NT : 4];  // see load_window
+    float4 plane[NT];               // half-pass: plane_vector of the chunk's items
+    float ref[OVERLAY ? (REF > UNITS ? REF : UNITS) : REF];
+    float unit_own[OVERLAY ? 1 : UNITS];
+    float cost[NT * 4];             // half-pass: neighbour costs, slot (thread << 2 | cand)
+    float2 stat[NT];                // half-pass: (mean, ssd) of each thread's pixel window
+    unsigned short items[NT * 4];   // half-pass: CTA item list, thread << 2 | cand
+    int warp_total[TH];
+    // Half-pass: cost of the chunk's item k at source s.
+    __device__ __forceinline__ float* unit(int s, int k) { return (OVERLAY ? ref : unit_own) + s * NT + k; }
 };
 
 template <int R, int ST, int NT>
@@ -396,162 +416,173 @@ __device__ __forceinline__ float source_cost(const Plane& P, cudaTextureObject_t
     return __fsub_rn(1.0f, ncc);
 }
 
-template <int R, int ST, int NT, int D>
-__device__ __forceinline__ float cost_f16(RefStats st, const __half2* s_win, const float* s_ref, int tw, int lx,
-                                          int ly, int x, int y, float d, float cnx, float cny, float cnz,
-                                          const ViewDesc* __restrict__ v, int topk, unsigned soft_mask) {
+// The plane (d, n) of pixel (x, y) as the homographies use it: m = K^-T n / (n.P)
+// with P = d K^-1 (x, y, 1), in xyz; w is 0 when |n.P| < 1e-8 (every cost is 2), else 1.
+__device__ __forceinline__ float4 plane_vector(const ViewDesc* __restrict__ v, int x, int y, float4 h) {
     const float* k = v->kinv;
+    const float d = h.x, cnx = h.y, cny = h.z, cnz = h.w;
     const float fx = static_cast<float>(x), fy = static_cast<float>(y);
     const float Px = __fmul_rn(d, __fmaf_rn(k[0], fx, __fmaf_rn(k[1], fy, k[2])));
     const float Py = __fmul_rn(d, __fmaf_rn(k[3], fx, __fmaf_rn(k[4], fy, k[5])));
     const float Pz = __fmul_rn(d, __fmaf_rn(k[6], fx, __fmaf_rn(k[7], fy, k[8])));
     const float ndp = __fmaf_rn(cnx, Px, __fmaf_rn(cny, Py, __fmul_rn(cnz, Pz)));
-    if (fabsf(ndp) < 1e-8f) return 2.0f;
+    if (fabsf(ndp) < 1e-8f) return make_float4(0.f, 0.f, 0.f, 0.f);
     const float ind = __frcp_rn(ndp);
-    const float m0 = __fmul_rn(__fmaf_rn(k[0], cnx, __fmaf_rn(k[3], cny, __fmul_rn(k[6], cnz))), ind);
-    const float m1 = __fmul_rn(__fmaf_rn(k[1], cnx, __fmaf_rn(k[4], cny, __fmul_rn(k[7], cnz))), ind);
-    const float m2 = __fmul_rn(__fmaf_rn(k[2], cnx, __fmaf_rn(k[5], cny, __fmul_rn(k[8], cnz))), ind);
+    return make_float4(__fmul_rn(__fmaf_rn(k[0], cnx, __fmaf_rn(k[3], cny, __fmul_rn(k[6], cnz))), ind),
+                       __fmul_rn(__fmaf_rn(k[1], cnx, __fmaf_rn(k[4], cny, __fmul_rn(k[7], cnz))), ind),
+                       __fmul_rn(__fmaf_rn(k[2], cnx, __fmaf_rn(k[5], cny, __fmul_rn(k[8], cnz))), ind), 1.0f);
+}
+
+// Cost of source s under the plane m (plane_vector) at pixel (x, y).
+template <int R, int ST, int NT, int D>
+__device__ __forceinline__ float unit_cost(const ViewDesc* __restrict__ v, int s, float m0, float m1, float m2,
+                                           RefStats st, const __half2* s_win, const float* s_ref, int tw, int lx,
+                                           int ly, int x, int y, unsigned soft_mask) {
     const float fW = static_cast<float>(v->W), fH = static_cast<float>(v->H);
     const float xa = static_cast<float>(x - R);
     const float ya = static_cast<float>(y - R);
-    float top0 = 2.0f, top1 = 2.0f, top2 = 2.0f;
-    const int S = v->S;
-    for (int s = 0; s < S; ++s) {
-        // A (9) and b (3) of the source: three 16-byte loads (ViewDesc::ab is 16-byte aligned).
-        const float4* A4 = reinterpret_cast<const float4*>(v->ab[s]);
-        const float4 q0 = __ldg(A4), q1 = __ldg(A4 + 1), q2 = __ldg(A4 + 2);
-        const float A[12] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w, q2.x, q2.y, q2.z, q2.w};
-        // Uniform over the launch: every lane of a warp takes the same sampler.
-        const bool soft = (soft_mask >> s) & 1u;
-        const float lo = soft ? 0.0f : 0.5f;  // texel-centre offset of the sampler's coordinate
-        Plane P;
-        P.h[6] = __fmaf_rn(A[11], m0, A[6]);
-        P.h[7] = __fmaf_rn(A[11], m1, A[7]);
-        P.h[8] = __fmaf_rn(A[11], m2, A[8]);
-        P.h[0] = __fmaf_rn(A[9], m0, A[0]);
-        P.h[1] = __fmaf_rn(A[9], m1, A[1]);
-        P.h[2] = __fmaf_rn(A[9], m2, A[2]);
-        P.h[3] = __fmaf_rn(A[10], m0, A[3]);
-        P.h[4] = __fmaf_rn(A[10], m1, A[4]);
-        P.h[5] = __fmaf_rn(A[10], m2, A[5]);
-        if (!soft) {  // texture taps: fold the +0.5 texel-centre offset into rows 0 and 1
-            P.h[0] = __fmaf_rn(0.5f, P.h[6], P.h[0]);
-            P.h[1] = __fmaf_rn(0.5f, P.h[7], P.h[1]);
-            P.h[2] = __fmaf_rn(0.5f, P.h[8], P.h[2]);
-            P.h[3] = __fmaf_rn(0.5f, P.h[6], P.h[3]);
-            P.h[4] = __fmaf_rn(0.5f, P.h[7], P.h[4]);
-            P.h[5] = __fmaf_rn(0.5f, P.h[8], P.h[5]);
-        }
-        // Corner test: in front of the source (w_z > 1e-6) with all four
-        // corners inside [lo, W - 1 + lo) x [lo, H - 1 + lo) by a 0.05 px
-        // margin, which covers the rounding of the row-stepped taps and of the
-        // corners themselves (stepped here from the first along the window's
-        // edges) where the homography is well conditioned (below).  The warp
-        // of the window rectangle is then the convex quad of its corners, so
-        // every tap is valid by the per-tap rules too.
-        const float ulo = __fadd_rn(lo, 0.05f), uhi = __fsub_rn(__fadd_rn(fW, lo), 1.05f);
-        const float vhi = __fsub_rn(__fadd_rn(fH, lo), 1.05f);
-        constexpr float SPAN = static_cast<float>((Win<R, ST>::SIDE - 1) * ST);
-        float cz[4], cx[4], cy[4];
-        cz[0] = __fmaf_rn(P.h[6], xa, __fmaf_rn(P.h[7], ya, P.h[8]));
-        cx[0] = __fmaf_rn(P.h[0], xa, __fmaf_rn(P.h[1], ya, P.h[2]));
-        cy[0] = __fmaf_rn(P.h[3], xa, __fmaf_rn(P.h[4], ya, P.h[5]));
-        cz[1] = __fmaf_rn(P.h[6], SPAN, cz[0]);
-        cx[1] = __fmaf_rn(P.h[0], SPAN, cx[0]);
-        cy[1] = __fmaf_rn(P.h[3], SPAN, cy[0]);
-        cz[2] = __fmaf_rn(P.h[7], SPAN, cz[0]);
-        cx[2] = __fmaf_rn(P.h[1], SPAN, cx[0]);
-        cy[2] = __fmaf_rn(P.h[4], SPAN, cy[0]);
-        cz[3] = __fmaf_rn(P.h[7], SPAN, cz[1]);
-        cx[3] = __fmaf_rn(P.h[1], SPAN, cx[1]);
-        cy[3] = __fmaf_rn(P.h[4], SPAN, cy[1]);
-        // Fully outside: in front at every corner and every corner beyond the
-        // same edge of the valid region by the margin.  The window's warp is
-        // the convex quad of its corners, so every tap is invalid, the count
-        // is 0 and the reference's rule makes the source cost 2 - no tap needs
-        // sampling.
-        const float olo = __fsub_rn(lo, 0.05f), ohi = __fadd_rn(__fadd_rn(fW, lo), -0.95f);
-        const float ovhi = __fadd_rn(__fadd_rn(fH, lo), -0.95f);
-        // Each corner is projected (approximate reciprocal, error far below the
-        // margin) and the tests run on the corners' bounding box: ~45
-        // instructions for the four corners instead of ~90 for per-corner
-        // products and compares.  A corner behind the camera fails `front`,
-        // and its garbage coordinates then decide nothing.
-        float umin = 0.f, umax = 0.f, vmin = 0.f, vmax = 0.f, zmin = 0.f;
+    // A (9) and b (3) of the source: three 16-byte loads (ViewDesc::ab is 16-byte aligned).
+    const float4* A4 = reinterpret_cast<const float4*>(v->ab[s]);
+    const float4 q0 = __ldg(A4), q1 = __ldg(A4 + 1), q2 = __ldg(A4 + 2);
+    const float A[12] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w, q2.x, q2.y, q2.z, q2.w};
+    // Uniform over the launch: every lane of a warp takes the same sampler.
+    const bool soft = (soft_mask >> s) & 1u;
+    const float lo = soft ? 0.0f : 0.5f;  // texel-centre offset of the sampler's coordinate
+    Plane P;
+    P.h[6] = __fmaf_rn(A[11], m0, A[6]);
+    P.h[7] = __fmaf_rn(A[11], m1, A[7]);
+    P.h[8] = __fmaf_rn(A[11], m2, A[8]);
+    P.h[0] = __fmaf_rn(A[9], m0, A[0]);
+    P.h[1] = __fmaf_rn(A[9], m1, A[1]);
+    P.h[2] = __fmaf_rn(A[9], m2, A[2]);
+    P.h[3] = __fmaf_rn(A[10], m0, A[3]);
+    P.h[4] = __fmaf_rn(A[10], m1, A[4]);
+    P.h[5] = __fmaf_rn(A[10], m2, A[5]);
+    if (!soft) {  // texture taps: fold the +0.5 texel-centre offset into rows 0 and 1
+        P.h[0] = __fmaf_rn(0.5f, P.h[6], P.h[0]);
+        P.h[1] = __fmaf_rn(0.5f, P.h[7], P.h[1]);
+        P.h[2] = __fmaf_rn(0.5f, P.h[8], P.h[2]);
+        P.h[3] = __fmaf_rn(0.5f, P.h[6], P.h[3]);
+        P.h[4] = __fmaf_rn(0.5f, P.h[7], P.h[4]);
+        P.h[5] = __fmaf_rn(0.5f, P.h[8], P.h[5]);
+    }
+    // Corner test: in front of the source (w_z > 1e-6) with all four
+    // corners inside [lo, W - 1 + lo) x [lo, H - 1 + lo) by a 0.05 px
+    // margin, which covers the rounding of the row-stepped taps and of the
+    // corners themselves (stepped here from the first along the window's
+    // edges) where the homography is well conditioned (below).  The warp
+    // of the window rectangle is then the convex quad of its corners, so
+    // every tap is valid by the per-tap rules too.
+    const float ulo = __fadd_rn(lo, 0.05f), uhi = __fsub_rn(__fadd_rn(fW, lo), 1.05f);
+    const float vhi = __fsub_rn(__fadd_rn(fH, lo), 1.05f);
+    constexpr float SPAN = static_cast<float>((Win<R, ST>::SIDE - 1) * ST);
+    float cz[4], cx[4], cy[4];
+    cz[0] = __fmaf_rn(P.h[6], xa, __fmaf_rn(P.h[7], ya, P.h[8]));
+    cx[0] = __fmaf_rn(P.h[0], xa, __fmaf_rn(P.h[1], ya, P.h[2]));
+    cy[0] = __fmaf_rn(P.h[3], xa, __fmaf_rn(P.h[4], ya, P.h[5]));
+    cz[1] = __fmaf_rn(P.h[6], SPAN, cz[0]);
+    cx[1] = __fmaf_rn(P.h[0], SPAN, cx[0]);
+    cy[1] = __fmaf_rn(P.h[3], SPAN, cy[0]);
+    cz[2] = __fmaf_rn(P.h[7], SPAN, cz[0]);
+    cx[2] = __fmaf_rn(P.h[1], SPAN, cx[0]);
+    cy[2] = __fmaf_rn(P.h[4], SPAN, cy[0]);
+    cz[3] = __fmaf_rn(P.h[7], SPAN, cz[1]);
+    cx[3] = __fmaf_rn(P.h[1], SPAN, cx[1]);
+    cy[3] = __fmaf_rn(P.h[4], SPAN, cy[1]);
+    // Fully outside: in front at every corner and every corner beyond the
+    // same edge of the valid region by the margin.  The window's warp is
+    // the convex quad of its corners, so every tap is invalid, the count
+    // is 0 and the reference's rule makes the source cost 2 - no tap needs
+    // sampling.
+    const float olo = __fsub_rn(lo, 0.05f), ohi = __fadd_rn(__fadd_rn(fW, lo), -0.95f);
+    const float ovhi = __fadd_rn(__fadd_rn(fH, lo), -0.95f);
+    // Each corner is projected (approximate reciprocal, error far below the
+    // margin) and the tests run on the corners' bounding box: ~45
+    // instructions for the four corners instead of ~90 for per-corner
+    // products and compares.  A corner behind the camera fails `front`,
+    // and its garbage coordinates then decide nothing.
+    float umin = 0.f, umax = 0.f, vmin = 0.f, vmax = 0.f, zmin = 0.f;
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            const float iz = rcp_approx(cz[c]);
-            const float2 uv = __fmul2_rn(make_float2(cx[c], cy[c]), make_float2(iz, iz));
-            if (c == 0) {
-                umin = umax = uv.x;
-                vmin = vmax = uv.y;
-                zmin = cz[c];
-            } else {
-                umin = fminf(umin, uv.x);
-                umax = fmaxf(umax, uv.x);
-                vmin = fminf(vmin, uv.y);
-                vmax = fmaxf(vmax, uv.y);
-                zmin = fminf(zmin, cz[c]);
-            }
-        }
-        // Conditioning.  The corners above and the row-stepped taps of
-        // source_cost evaluate the homography in different orders, so their
-        // rounding differs: by at most (SIDE + 5) roundings of the largest
-        // partial sum, Mx = |h0| X1 + |h1| Y1 + |h2| for w_x (X1, Y1 bound the
-        // window's absolute pixel coordinates), likewise My and Mz.  In the
-        // projected coordinate that is (Mx + |u| Mz) (SIDE + 5) 2^-24 / z_min.
-        // A plane seen nearly edge-on makes the terms large and cancelling,
-        // and the corners can then pass the test while a tap falls outside
-        // the source.  The decision stands only while the bound (with |u|
-        // taken as at least 1, which also bounds the error of z) stays within
-        // 0.04 px of the 0.05 px margin; other windows take the per-tap
-        // checked form, which gives the same bits whenever every tap is valid.
-        // NaN or infinite corners fail the comparison too.  COND counts one
-        // rounding more than the bound above, for slack.
-        constexpr float COND = 0.04f / ((Win<R, ST>::SIDE + 6) * 5.9604645e-8f);
-        const float X1 = fabsf(xa) + SPAN, Y1 = fabsf(ya) + SPAN;
-        const float Mx = __fmaf_rn(fabsf(P.h[0]), X1, __fmaf_rn(fabsf(P.h[1]), Y1, fabsf(P.h[2])));
-        const float My = __fmaf_rn(fabsf(P.h[3]), X1, __fmaf_rn(fabsf(P.h[4]), Y1, fabsf(P.h[5])));
-        const float Mz = __fmaf_rn(fabsf(P.h[6]), X1, __fmaf_rn(fabsf(P.h[7]), Y1, fabsf(P.h[8])));
-        const float Ua = fmaxf(1.0f, fmaxf(fabsf(umin), fabsf(umax)));
-        const float Va = fmaxf(1.0f, fmaxf(fabsf(vmin), fabsf(vmax)));
-        const float zc = __fmul_rn(zmin, COND);
-        const bool front = zmin > 1e-6f && __fmaf_rn(Ua, Mz, Mx) <= zc && __fmaf_rn(Va, Mz, My) <= zc;
-        // SOFT_MASK_CHECKED (self-checking builds only, uniform over the
-        // launch) turns both shortcuts off, to test that they change no result.
-#ifdef HP_SELF_CHECK
-        const bool shortcuts = (soft_mask & SOFT_MASK_CHECKED) == 0u;
-#else
-        constexpr bool shortcuts = true;
-#endif
-        const bool inside = front && umin >= ulo && umax < uhi && vmin >= ulo && vmax < vhi;
-        const bool left = umax < olo, right = umin >= ohi, top = vmax < olo, bottom = vmin >= ovhi;
-        const bool outside = shortcuts && front && (left || right || top || bottom);
-        // One form per warp for the lanes that sample: the checked form gives
-        // the unchecked form's bits whenever every tap is valid, so lanes that
-        // are inside lose nothing.
-        const bool all_inside = shortcuts && __all_sync(__activemask(), inside || outside);
-        float c = 2.0f;
-        if (outside) {
-        } else if (soft) {
-#ifdef HP_COUNT_TAPS
-            atomicAdd(&g_taps, static_cast<unsigned long long>(Win<R, ST>::N));
-#endif
-            const uint2* qb = soft_base(v->src_quad[s]);
-            c = all_inside ? source_cost<R, ST, false, true, NT, D>(P, 0, qb, st, s_win, s_ref, tw, lx, ly, x,
-                                                             y, fW, fH)
-                           : source_cost<R, ST, true, true, NT, D>(P, 0, qb, st, s_win, s_ref, tw, lx, ly, x,
-                                                            y, fW, fH);
+    for (int c = 0; c < 4; ++c) {
+        const float iz = rcp_approx(cz[c]);
+        const float2 uv = __fmul2_rn(make_float2(cx[c], cy[c]), make_float2(iz, iz));
+        if (c == 0) {
+            umin = umax = uv.x;
+            vmin = vmax = uv.y;
+            zmin = cz[c];
         } else {
-#ifdef HP_COUNT_TAPS
-            atomicAdd(&g_taps, static_cast<unsigned long long>(Win<R, ST>::N));
-#endif
-            const cudaTextureObject_t tex = v->src_tex16[s];
-            c = all_inside ? source_cost<R, ST, false, false, NT, D>(P, tex, nullptr, st, s_win, s_ref, tw, lx, ly, x, y,
-                                                              fW, fH)
-                           : source_cost<R, ST, true, false, NT, D>(P, tex, nullptr, st, s_win, s_ref, tw, lx, ly, x, y,
-                                                             fW, fH);
+            umin = fminf(umin, uv.x);
+            umax = fmaxf(umax, uv.x);
+            vmin = fminf(vmin, uv.y);
+            vmax = fmaxf(vmax, uv.y);
+            zmin = fminf(zmin, cz[c]);
         }
+    }
+    // Conditioning.  The corners above and the row-stepped taps of
+    // source_cost evaluate the homography in different orders, so their
+    // rounding differs: by at most (SIDE + 5) roundings of the largest
+    // partial sum, Mx = |h0| X1 + |h1| Y1 + |h2| for w_x (X1, Y1 bound the
+    // window's absolute pixel coordinates), likewise My and Mz.  In the
+    // projected coordinate that is (Mx + |u| Mz) (SIDE + 5) 2^-24 / z_min.
+    // A plane seen nearly edge-on makes the terms large and cancelling,
+    // and the corners can then pass the test while a tap falls outside
+    // the source.  The decision stands only while the bound (with |u|
+    // taken as at least 1, which also bounds the error of z) stays within
+    // 0.04 px of the 0.05 px margin; other windows take the per-tap
+    // checked form, which gives the same bits whenever every tap is valid.
+    // NaN or infinite corners fail the comparison too.  COND counts one
+    // rounding more than the bound above, for slack.
+    constexpr float COND = 0.04f / ((Win<R, ST>::SIDE + 6) * 5.9604645e-8f);
+    const float X1 = fabsf(xa) + SPAN, Y1 = fabsf(ya) + SPAN;
+    const float Mx = __fmaf_rn(fabsf(P.h[0]), X1, __fmaf_rn(fabsf(P.h[1]), Y1, fabsf(P.h[2])));
+    const float My = __fmaf_rn(fabsf(P.h[3]), X1, __fmaf_rn(fabsf(P.h[4]), Y1, fabsf(P.h[5])));
+    const float Mz = __fmaf_rn(fabsf(P.h[6]), X1, __fmaf_rn(fabsf(P.h[7]), Y1, fabsf(P.h[8])));
+    const float Ua = fmaxf(1.0f, fmaxf(fabsf(umin), fabsf(umax)));
+    const float Va = fmaxf(1.0f, fmaxf(fabsf(vmin), fabsf(vmax)));
+    const float zc = __fmul_rn(zmin, COND);
+    const bool front = zmin > 1e-6f && __fmaf_rn(Ua, Mz, Mx) <= zc && __fmaf_rn(Va, Mz, My) <= zc;
+    // SOFT_MASK_CHECKED (self-checking builds only, uniform over the
+    // launch) turns both shortcuts off, to test that they change no result.
+#ifdef HP_SELF_CHECK
+    const bool shortcuts = (soft_mask & SOFT_MASK_CHECKED) == 0u;
+#else
+    constexpr bool shortcuts = true;
+#endif
+    const bool inside = front && umin >= ulo && umax < uhi && vmin >= ulo && vmax < vhi;
+    const bool left = umax < olo, right = umin >= ohi, top = vmax < olo, bottom = vmin >= ovhi;
+    const bool outside = shortcuts && front && (left || right || top || bottom);
+    // One form per warp for the lanes that sample: the checked form gives
+    // the unchecked form's bits whenever every tap is valid, so lanes that
+    // are inside lose nothing.
+    const bool all_inside = shortcuts && __all_sync(__activemask(), inside || outside);
+    float c = 2.0f;
+    if (outside) {
+    } else if (soft) {
+#ifdef HP_COUNT_TAPS
+        atomicAdd(&g_taps, static_cast<unsigned long long>(Win<R, ST>::N));
+#endif
+        const uint2* qb = soft_base(v->src_quad[s]);
+        c = all_inside ? source_cost<R, ST, false, true, NT, D>(P, 0, qb, st, s_win, s_ref, tw, lx, ly, x,
+                                                         y, fW, fH)
+                       : source_cost<R, ST, true, true, NT, D>(P, 0, qb, st, s_win, s_ref, tw, lx, ly, x,
+                                                        y, fW, fH);
+    } else {
+#ifdef HP_COUNT_TAPS
+        atomicAdd(&g_taps, static_cast<unsigned long long>(Win<R, ST>::N));
+#endif
+        const cudaTextureObject_t tex = v->src_tex16[s];
+        c = all_inside ? source_cost<R, ST, false, false, NT, D>(P, tex, nullptr, st, s_win, s_ref, tw, lx, ly, x, y,
+                                                          fW, fH)
+                       : source_cost<R, ST, true, false, NT, D>(P, tex, nullptr, st, s_win, s_ref, tw, lx, ly, x, y,
+                                                         fW, fH);
+    }
+    return c;
+}
+
+// Mean of the min(topk, S) lowest source costs, inserted one by one.
+struct Lowest {
+    float top0 = 2.0f, top1 = 2.0f, top2 = 2.0f;
+    __device__ __forceinline__ void insert(float c) {
         if (c < top2) {
             top2 = c;
             if (top2 < top1) {
@@ -560,17 +591,26 @@ __device__ __forceinline__ float cost_f16(RefStats st, const __half2* s_win, con
             }
         }
     }
-    const int kk = min(topk, S);
-    float sum = top0;
-    if (kk > 1) sum = __fadd_rn(sum, top1);
-    if (kk > 2) sum = __fadd_rn(sum, top2);
-    return __fdiv_rn(sum, static_cast<float>(kk));
+    __device__ __forceinline__ float mean(int kk) const {
+        float sum = top0;
+        if (kk > 1) sum = __fadd_rn(sum, top1);
+        if (kk > 2) sum = __fadd_rn(sum, top2);
+        return __fdiv_rn(sum, static_cast<float>(kk));
+    }
+};
+
+extern __shared__ __align__(16) unsigned char dynamic_smem[];
+template <int R, int ST, int TH>
+__device__ __forceinline__ Shared<R, ST, TH>& shared_of() {
+    return *reinterpret_cast<Shared<R, ST, TH>*>(dynamic_smem);
 }
 
 template <int R, int ST, int TH, int D>
 __device__ __forceinline__ void tile_cost16(const ViewDesc* v, int tile_x, int tile_y, const SolveConsts& sc,
-                                            float* s_ref, __half2* s_win) {
+                                            Shared<R, ST, TH>& sm) {
     constexpr int NT = Tile<TH>::NT;
+    float* s_ref = sm.ref;
+    __half2* s_win = sm.win;
     constexpr int tw = TILE_W + 2 * R, th = TH + 2 * R;
     const int x0 = tile_x * TILE_W, y0 = tile_y * TH;
     load_ref_tile16<NT>(s_ref, tw, th, v, x0, y0, R);
@@ -578,62 +618,59 @@ __device__ __forceinline__ void tile_cost16(const ViewDesc* v, int tile_x, int t
     const int ly = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int y = y0 + ly;
     if (y >= v->H) return;
+    // Lanes own consecutive pixels (two 32-pixel halves of the tile row): a
+    // warp's taps of one window position then lie next to each other.
     for (int j = 0; j < 2; ++j) {
-        const int lx = 2 * lane + j, x = x0 + lx;
+        const int lx = 32 * j + lane, x = x0 + lx;
         if (x >= v->W) continue;
         const RefStats st = load_window<R, ST, NT>(s_win, s_ref, tw, lx, ly);
         const size_t idx = static_cast<size_t>(y) * v->W + x;
-        const float4 h = v->hyp[idx];
-        v->cost[idx] = cost_f16<R, ST, NT, D>(st, s_win + threadIdx.x * Win<R, ST>::VEC, s_ref, tw, lx, ly, x, y, h.x, h.y, h.z, h.w, v,
-                                       sc.top_k, sc.soft_mask);
+        const float4 m = plane_vector(v, x, y, v->hyp[idx]);
+        Lowest low;
+        if (m.w != 0.0f)
+            for (int s = 0; s < v->S; ++s)
+                low.insert(unit_cost<R, ST, NT, D>(v, s, m.x, m.y, m.z, st,
+                                                   s_win + threadIdx.x * Win<R, ST>::VEC, s_ref, tw, lx, ly, x, y,
+                                                   sc.soft_mask));
+        v->cost[idx] = low.mean(min(sc.top_k, v->S));
     }
 }
 
 template <int R, int ST, int TH, int D>
 __global__ void __launch_bounds__(Tile<TH>::NT, Tile<TH>::MIN_BLOCKS) cost16_kernel(BatchList bl, SolveConsts sc) {
-    __shared__ float s_ref[(TILE_W + 2 * R) * (TH + 2 * R)];
-    __shared__ __align__(16) __half2 s_win[Win<R, ST>::IN_SMEM ? WIN_PAIRS_MAX * Tile<TH>::NT : 1];
     int tile_x, tile_y;
     const ViewDesc* v = locate_tile16(bl, blockIdx.x, &tile_x, &tile_y);
-    tile_cost16<R, ST, TH, D>(v, tile_x, tile_y, sc, s_ref, s_win);
+    tile_cost16<R, ST, TH, D>(v, tile_x, tile_y, sc, shared_of<R, ST, TH>());
 }
 
-// One red-black half-pass.  The neighbour phase is compacted across the CTA:
-// every lane lists the neighbour planes its pixel must score (duplicates of
-// the current plane or of an earlier neighbour skipped), the lists of all
-// eight warps are concatenated in shared memory, and the warps score the
-// union 32 items at a time (warp w takes items [32 (w + 8 k), 32 (w + 8 k) +
-// 32)).  An item reads its owner pixel's window statistics and s_win column
-// from shared memory and leaves its cost in the owner's slot, so owners then
-// fold the costs in L, R, U, D order exactly as if they had scored them
-// themselves: results do not depend on which lane scored what.
-// Shared memory of the half-pass beyond the reference tile and window (TH warps).
-template <int TH>
-struct PassSmem {
-    float cost[TH][32 * 4];           // neighbour cost, slot (lane << 2 | cand) of the owner's warp
-    unsigned short items[TH * 128];   // CTA item list: warp << 7 | lane << 2 | cand
-    float2 stat[32 * TH];             // (mean, ssd) of each thread's pixel window
-    int warp_total[TH];
-};
-
+// One red-black half-pass.  Scoring is split into units of (item, source): an
+// item is a pixel with a plane to score, and the CTA's threads take the units
+// of up to NT items in order (unit u: item u % n, source u / n), so every warp
+// has full lanes whatever the number of items and whatever sources each warp
+// would have drawn.  Scored in rounds: the neighbour planes of all pixels of
+// the tile (every lane lists the ones its pixel must score, the lists of all
+// warps concatenated), then one round per refinement step with one perturbed
+// plane per pixel.  A unit reads its pixel's window statistics and s_win
+// column from shared memory; owners fold their costs in L, R, U, D order
+// exactly as if they had scored them themselves, so results do not depend on
+// which lane scored what.
 template <int R, int ST, int TH, int D>
 __device__ __forceinline__ void tile_propagate16(const ViewDesc* v, int tile_x, int tile_y, const SolveConsts& sc,
-                                                 int iteration, int color, float* s_ref, __half2* s_win,
-                                                 PassSmem<TH>& sm) {
+                                                 int iteration, int color, Shared<R, ST, TH>& sm) {
     constexpr int NT = Tile<TH>::NT, WARPS = TH;
+    float* s_ref = sm.ref;
+    __half2* s_win = sm.win;
     constexpr int tw = TILE_W + 2 * R, th = TH + 2 * R;
     const int x0 = tile_x * TILE_W, y0 = tile_y * TH;
     load_ref_tile16<NT>(s_ref, tw, th, v, x0, y0, R);
     __syncthreads();
-    const int W = v->W, H = v->H;
-    const int ly = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int W = v->W, H = v->H, S = v->S;
+    const int tid = threadIdx.x, ly = tid >> 5, lane = tid & 31;
     const int y = y0 + ly;
-    const int parity = (y + color) & 1;
-    const int lx = 2 * lane + parity;
+    const int lx = 2 * lane + ((y + color) & 1);
     const int x = x0 + lx;
     const bool active = y < H && x < W;  // every thread takes part in the CTA barriers below
     const size_t idx = static_cast<size_t>(y) * W + x;
-    const float dmin = v->dmin, dmax = v->dmax;
     RefStats st{0.f, 0.f};
     float4 best = make_float4(0.f, 0.f, 0.f, 0.f);
     float best_cost = 0.f;
@@ -645,7 +682,7 @@ __device__ __forceinline__ void tile_propagate16(const ViewDesc* v, int tile_x, 
         best_cost = cost_value(v->cost[idx]);
         need = neighbour_needs(v, x, y, best, sc.memo && iteration > 0);
     }
-    sm.stat[threadIdx.x] = make_float2(st.mean, st.ssd);
+    sm.stat[tid] = make_float2(st.mean, st.ssd);
     const int cnt = __popc(need);
     int incl = cnt;
 #pragma unroll
@@ -655,80 +692,110 @@ __device__ __forceinline__ void tile_propagate16(const ViewDesc* v, int tile_x, 
     }
     if (lane == 31) sm.warp_total[ly] = incl;
     __syncthreads();  // warp totals, window statistics and s_win columns are complete
-    int offset = 0, total = 0;
-#pragma unroll
-    for (int w = 0; w < WARPS; ++w) {
-        const int t = sm.warp_total[w];
-        offset += w < ly ? t : 0;
-        total += t;
-    }
+    int total = 0;
     {
-        int k = offset + incl - cnt;
+        int k = incl - cnt;
+#pragma unroll
+        for (int w = 0; w < WARPS; ++w) {
+            const int t = sm.warp_total[w];
+            k += w < ly ? t : 0;
+            total += t;
+        }
         for (int cand = 0; cand < 4; ++cand)
-            if (need & (1u << cand)) sm.items[k++] = static_cast<unsigned short>((ly << 7) | (lane << 2) | cand);
+            if (need & (1u << cand)) sm.items[k++] = static_cast<unsigned short>((tid << 2) | cand);
     }
     __syncthreads();  // the CTA's item list is complete
-    for (int base = ly * 32; base < total; base += NT) {
-        const int w = base + lane;
-        if (w < total) {
-            const int item = sm.items[w];
-            const int oly = item >> 7, owner = (item >> 2) & 31, cand = item & 3;
-            const int oy = y0 + oly, olx = 2 * owner + ((oy + color) & 1), ox = x0 + olx;
-            const float2 os = sm.stat[oly * 32 + owner];
-            const int nxp = ox + (cand == 0 ? -1 : (cand == 1 ? 1 : 0));
-            const int nyp = oy + (cand == 2 ? -1 : (cand == 3 ? 1 : 0));
-            if (!HP_CHECK(nxp >= 0 && nxp < W && nyp >= 0 && nyp < H, HP_CHECK_NEIGHBOUR, ox, oy, nxp, nyp, W, H,
-                          0.f, 0.f, 0.f, 0.f))
-                continue;
-            const float4 h = v->hyp[static_cast<size_t>(nyp) * W + nxp];
-            sm.cost[oly][item & 127] = cost_f16<R, ST, NT, D>(RefStats{os.x, os.y}, s_win + (oly * 32 + owner) * Win<R, ST>::VEC, s_ref, tw,
-                                                       olx, oly, ox, oy, h.x, h.y, h.z, h.w, v, sc.top_k,
-                                                       sc.soft_mask);
-        }
-    }
-    __syncthreads();  // every neighbour cost is in its owner's slot
-    if (!active) return;
-#pragma unroll
-    for (int cand = 0; cand < 4; ++cand) {
-        if (need & (1u << cand)) {
-            const float c = sm.cost[ly][(lane << 2) | cand];
-            if (c < best_cost) {
-                const int nxp = x + (cand == 0 ? -1 : (cand == 1 ? 1 : 0));
-                const int nyp = y + (cand == 2 ? -1 : (cand == 3 ? 1 : 0));
-                best_cost = c;
-                settled = false;
-                best = v->hyp[static_cast<size_t>(nyp) * W + nxp];
-            }
-        }
-    }
-    const float3 ray = view_ray(v->kinv, x, y);
-    float drange = __fmul_rn(__fsub_rn(dmax, dmin), 0.5f);
+    float drange = __fmul_rn(__fsub_rn(v->dmax, v->dmin), 0.5f);
     float nrange = 1.0f;
     for (int i = 0; i < iteration; ++i) {
         drange = __fmul_rn(drange, sc.iter_decay);
         nrange = __fmul_rn(nrange, sc.iter_decay);
     }
-    for (int step = 0; step < sc.refine_steps; ++step) {
-        const uint4 rr = philox4x32_10(make_uint4(static_cast<uint32_t>(idx), v->view_id,
-                                                  1u + static_cast<uint32_t>(iteration), static_cast<uint32_t>(step)),
-                                       v->seed_lo, v->seed_hi);
-        float cd = __fmaf_rn(__fmaf_rn(u01(rr.x), 2.0f, -1.0f), drange, best.x);
-        cd = fmaxf(dmin, fminf(dmax, cd));
-        const float cx = __fmaf_rn(__fmaf_rn(u01(rr.y), 2.0f, -1.0f), nrange, best.y);
-        const float cy = __fmaf_rn(__fmaf_rn(u01(rr.z), 2.0f, -1.0f), nrange, best.z);
-        const float cz = __fmaf_rn(__fmaf_rn(u01(rr.w), 2.0f, -1.0f), nrange, best.w);
-        float3 cn = normalize3_rn(cx, cy, cz);
-        if (dot3_rn(cn, ray) > 0.0f) cn = make_float3(-cn.x, -cn.y, -cn.z);
-        const float c = cost_f16<R, ST, NT, D>(st, s_win + threadIdx.x * Win<R, ST>::VEC, s_ref, tw, lx, ly, x, y, cd, cn.x, cn.y, cn.z, v,
-                                        sc.top_k, sc.soft_mask);
-        if (c < best_cost) {
+#pragma unroll 1
+    for (int round = 0; round <= sc.refine_steps; ++round) {
+        float4 trial = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (round > 0) {
+            if (active) {
+                const uint4 rr =
+                    philox4x32_10(make_uint4(static_cast<uint32_t>(idx), v->view_id,
+                                             1u + static_cast<uint32_t>(iteration), static_cast<uint32_t>(round - 1)),
+                                  v->seed_lo, v->seed_hi);
+                const float cd = __fmaf_rn(__fmaf_rn(u01(rr.x), 2.0f, -1.0f), drange, best.x);
+                const float cx = __fmaf_rn(__fmaf_rn(u01(rr.y), 2.0f, -1.0f), nrange, best.y);
+                const float cy = __fmaf_rn(__fmaf_rn(u01(rr.z), 2.0f, -1.0f), nrange, best.z);
+                const float cz = __fmaf_rn(__fmaf_rn(u01(rr.w), 2.0f, -1.0f), nrange, best.w);
+                float3 cn = normalize3_rn(cx, cy, cz);
+                if (dot3_rn(cn, view_ray(v->kinv, x, y)) > 0.0f) cn = make_float3(-cn.x, -cn.y, -cn.z);
+                trial = make_float4(fmaxf(v->dmin, fminf(v->dmax, cd)), cn.x, cn.y, cn.z);
+            }
+            drange = __fmul_rn(drange, sc.step_decay);
+            nrange = __fmul_rn(nrange, sc.step_decay);
+        }
+        const int count = round == 0 ? total : NT;
+        float c = 2.0f;
+#pragma unroll 1
+        for (int c0 = 0; c0 < count; c0 += NT) {
+            const int n = min(NT, count - c0);
+            int item = tid << 2;
+            float4 m = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (round > 0) {
+                if (active) m = plane_vector(v, x, y, trial);
+            } else if (tid < n) {
+                item = sm.items[c0 + tid];
+                const int o = item >> 2, cand = item & 3;
+                const int oy = y0 + (o >> 5), ox = x0 + 2 * (o & 31) + ((oy + color) & 1);
+                const int nxp = ox + (cand == 0 ? -1 : (cand == 1 ? 1 : 0));
+                const int nyp = oy + (cand == 2 ? -1 : (cand == 3 ? 1 : 0));
+                if (HP_CHECK(nxp >= 0 && nxp < W && nyp >= 0 && nyp < H, HP_CHECK_NEIGHBOUR, ox, oy, nxp, nyp, W, H,
+                             0.f, 0.f, 0.f, 0.f))
+                    m = plane_vector(v, ox, oy, v->hyp[static_cast<size_t>(nyp) * W + nxp]);
+            }
+            sm.plane[tid] = m;
+            __syncthreads();  // the chunk's planes are complete
+#pragma unroll 1
+            for (int u = tid; u < n * S; u += NT) {
+                const int s = u / n, k = u - s * n;
+                const int o = round == 0 ? sm.items[c0 + k] >> 2 : k;
+                const int oly = o >> 5, oy = y0 + oly, olx = 2 * (o & 31) + ((oy + color) & 1);
+                const float2 os = sm.stat[o];
+                const float4 um = sm.plane[k];
+                float uc = 2.0f;
+                if (um.w != 0.0f)
+                    uc = unit_cost<R, ST, NT, D>(v, s, um.x, um.y, um.z, RefStats{os.x, os.y},
+                                                 s_win + o * Win<R, ST>::VEC, s_ref, tw, olx, oly, x0 + olx, oy,
+                                                 sc.soft_mask);
+                *sm.unit(s, k) = uc;
+            }
+            __syncthreads();  // the chunk's source costs are complete
+            if (tid < n) {
+                Lowest low;
+                for (int s = 0; s < S; ++s) low.insert(*sm.unit(s, tid));
+                c = low.mean(min(sc.top_k, S));
+                if (round == 0) sm.cost[item] = c;
+            }
+        }
+        if (round == 0) {
+            __syncthreads();  // every neighbour cost is in its owner's slot
+#pragma unroll
+            for (int cand = 0; cand < 4; ++cand) {
+                if (need & (1u << cand)) {
+                    const float nc = sm.cost[(tid << 2) | cand];
+                    if (nc < best_cost) {
+                        const int nxp = x + (cand == 0 ? -1 : (cand == 1 ? 1 : 0));
+                        const int nyp = y + (cand == 2 ? -1 : (cand == 3 ? 1 : 0));
+                        best_cost = nc;
+                        settled = false;
+                        best = v->hyp[static_cast<size_t>(nyp) * W + nxp];
+                    }
+                }
+            }
+        } else if (active && c < best_cost) {
             best_cost = c;
             settled = false;
-            best = make_float4(cd, cn.x, cn.y, cn.z);
+            best = trial;
         }
-        drange = __fmul_rn(drange, sc.step_decay);
-        nrange = __fmul_rn(nrange, sc.step_decay);
     }
+    if (!active) return;
     v->hyp[idx] = best;
     v->cost[idx] = sc.memo && settled ? -best_cost : best_cost;
 }
@@ -736,21 +803,16 @@ __device__ __forceinline__ void tile_propagate16(const ViewDesc* v, int tile_x, 
 template <int R, int ST, int TH, int D>
 __global__ void __launch_bounds__(Tile<TH>::NT, Tile<TH>::MIN_BLOCKS) propagate16_kernel(BatchList bl, SolveConsts sc,
                                                                                        int iteration, int color) {
-    __shared__ float s_ref[(TILE_W + 2 * R) * (TH + 2 * R)];
-    __shared__ __align__(16) __half2 s_win[Win<R, ST>::IN_SMEM ? WIN_PAIRS_MAX * Tile<TH>::NT : 1];
-    __shared__ PassSmem<TH> sm;
     int tile_x, tile_y;
     const ViewDesc* v = locate_tile16(bl, blockIdx.x, &tile_x, &tile_y);
-    tile_propagate16<R, ST, TH, D>(v, tile_x, tile_y, sc, iteration, color, s_ref, s_win, sm);
+    tile_propagate16<R, ST, TH, D>(v, tile_x, tile_y, sc, iteration, color, shared_of<R, ST, TH>());
 }
 
 // Persistent form (see Schedule and the FP32 persistent kernel): the stage
 // bodies are those of the per-stage kernels, so the results are bit-identical.
 template <int R, int ST, int TH, int D>
 __global__ void __launch_bounds__(Tile<TH>::NT, Tile<TH>::MIN_BLOCKS) persistent16_kernel(Schedule s) {
-    __shared__ float s_ref[(TILE_W + 2 * R) * (TH + 2 * R)];
-    __shared__ __align__(16) __half2 s_win[Win<R, ST>::IN_SMEM ? WIN_PAIRS_MAX * Tile<TH>::NT : 1];
-    __shared__ PassSmem<TH> sm;
+    Shared<R, ST, TH>& sm = shared_of<R, ST, TH>();
     // The claimed tile lives in shared memory: thread 0 decodes it once and
     // publishes it after the stage, so no thread carries it through the body.
     __shared__ SchedTile s_tile;
@@ -781,10 +843,10 @@ __global__ void __launch_bounds__(Tile<TH>::NT, Tile<TH>::MIN_BLOCKS) persistent
         if (stage == 0) {
             tile_init(v, tx, ty);
             __syncthreads();
-            tile_cost16<R, ST, TH, D>(v, tx, ty, s.sc, s_ref, s_win);
+            tile_cost16<R, ST, TH, D>(v, tx, ty, s.sc, sm);
         } else if (stage <= 2 * v->iterations) {
             const int k = stage - 1;
-            tile_propagate16<R, ST, TH, D>(v, tx, ty, s.sc, k >> 1, k & 1, s_ref, s_win, sm);
+            tile_propagate16<R, ST, TH, D>(v, tx, ty, s.sc, k >> 1, k & 1, sm);
         } else if (is_filter_stage(v, stage)) {
             tile_filter(s.views, v, tx, ty, true);  // geometric check, then the maps
         } else {
@@ -805,13 +867,24 @@ struct Dispatch {
     static cudaError_t run(int mode, const BatchList* bl, const SolveConsts& sc, int iteration, int color,
                            const Schedule* s, int grid, cudaStream_t st, int* occ) {
         constexpr int NT = Tile<TH>::NT;
+        constexpr int smem = static_cast<int>(sizeof(Shared<R, ST, TH>));
+        // Opt in to more than 48 KB on the current device (a property of the function there; setting it again
+        // is harmless).
+        auto allow = [](const void* f) {
+            return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        };
+        cudaError_t e;
         if (mode == 2) {
-            if (occ) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, persistent16_kernel<R, ST, TH, D>, NT, 0);
-            persistent16_kernel<R, ST, TH, D><<<grid, NT, 0, st>>>(*s);
+            if ((e = allow(reinterpret_cast<const void*>(persistent16_kernel<R, ST, TH, D>))) != cudaSuccess) return e;
+            if (occ)
+                return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, persistent16_kernel<R, ST, TH, D>, NT, smem);
+            persistent16_kernel<R, ST, TH, D><<<grid, NT, smem, st>>>(*s);
         } else if (mode == 0) {
-            cost16_kernel<R, ST, TH, D><<<bl->total_tiles, NT, 0, st>>>(*bl, sc);
+            if ((e = allow(reinterpret_cast<const void*>(cost16_kernel<R, ST, TH, D>))) != cudaSuccess) return e;
+            cost16_kernel<R, ST, TH, D><<<bl->total_tiles, NT, smem, st>>>(*bl, sc);
         } else {
-            propagate16_kernel<R, ST, TH, D><<<bl->total_tiles, NT, 0, st>>>(*bl, sc, iteration, color);
+            if ((e = allow(reinterpret_cast<const void*>(propagate16_kernel<R, ST, TH, D>))) != cudaSuccess) return e;
+            propagate16_kernel<R, ST, TH, D><<<bl->total_tiles, NT, smem, st>>>(*bl, sc, iteration, color);
         }
         return cudaGetLastError();
     }
