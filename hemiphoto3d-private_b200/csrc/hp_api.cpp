@@ -150,6 +150,7 @@ hp_status fill_desc(hp_ctx* ctx, const hp_job* j, int jobno, hp::ViewDesc* d, in
         for (int s = 0; s < j->num_sources; ++s)
             for (int i = 0; i < 12; ++i) d->ab[s][i] = static_cast<float>(ab[12 * s + i]);
     }
+    hp::order_sources(d);
     d->tile_h = tile_h;
     d->tiles_x = (ref.W + hp::TILE_W - 1) / hp::TILE_W;
     d->tiles_y = (ref.H + tile_h - 1) / tile_h;

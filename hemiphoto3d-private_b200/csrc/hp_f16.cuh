@@ -121,6 +121,7 @@ struct alignas(16) Shared {
     float2 stat[NT];                // half-pass: (mean, ssd) of each thread's pixel window
     unsigned short items[NT * 4];   // half-pass: CTA item list, thread << 2 | cand
     int warp_total[TH];
+    int survivors;                  // half-pass: entries of the refinement round's second list
     // Half-pass: cost of the chunk's item k at source s.
     __device__ __forceinline__ float* unit(int s, int k) { return (OVERLAY ? ref : unit_own) + s * NT + k; }
 };
@@ -705,6 +706,7 @@ __device__ __forceinline__ void tile_propagate16(const ViewDesc* v, int tile_x, 
             if (need & (1u << cand)) sm.items[k++] = static_cast<unsigned short>((tid << 2) | cand);
     }
     __syncthreads();  // the CTA's item list is complete
+    const int kk = min(sc.top_k, S), lead = S - kk + 1;
     float drange = __fmul_rn(__fsub_rn(v->dmax, v->dmin), 0.5f);
     float nrange = 1.0f;
     for (int i = 0; i < iteration; ++i) {
@@ -733,6 +735,7 @@ __device__ __forceinline__ void tile_propagate16(const ViewDesc* v, int tile_x, 
         }
         const int count = round == 0 ? total : NT;
         float c = 2.0f;
+        bool keep = true;
 #pragma unroll 1
         for (int c0 = 0; c0 < count; c0 += NT) {
             const int n = min(NT, count - c0);
@@ -751,26 +754,51 @@ __device__ __forceinline__ void tile_propagate16(const ViewDesc* v, int tile_x, 
                     m = plane_vector(v, ox, oy, v->hyp[static_cast<size_t>(nyp) * W + nxp]);
             }
             sm.plane[tid] = m;
+            if (tid == 0) sm.survivors = 0;
             __syncthreads();  // the chunk's planes are complete
+            // Sources first .. last - 1 of the view's order, for the chunk's items (a refinement round's second
+            // part: for the listed survivors).
+            int units = n, first = 0, last = round == 0 ? S : lead;
 #pragma unroll 1
-            for (int u = tid; u < n * S; u += NT) {
-                const int s = u / n, k = u - s * n;
-                const int o = round == 0 ? sm.items[c0 + k] >> 2 : k;
-                const int oly = o >> 5, oy = y0 + oly, olx = 2 * (o & 31) + ((oy + color) & 1);
-                const float2 os = sm.stat[o];
-                const float4 um = sm.plane[k];
-                float uc = 2.0f;
-                if (um.w != 0.0f)
-                    uc = unit_cost<R, ST, NT, D>(v, s, um.x, um.y, um.z, RefStats{os.x, os.y},
-                                                 s_win + o * Win<R, ST>::VEC, s_ref, tw, olx, oly, x0 + olx, oy,
-                                                 sc.soft_mask);
-                *sm.unit(s, k) = uc;
+            for (;;) {
+#pragma unroll 1
+                for (int u = tid; u < units * (last - first); u += NT) {
+                    const int q = u / units;
+                    int k = u - q * units;
+                    if (first > 0) k = sm.items[k];
+                    const int o = round == 0 ? sm.items[c0 + k] >> 2 : k;
+                    const int oly = o >> 5, oy = y0 + oly, olx = 2 * (o & 31) + ((oy + color) & 1);
+                    const float2 os = sm.stat[o];
+                    const float4 um = sm.plane[k];
+                    float uc = 2.0f;
+                    if (um.w != 0.0f)
+                        uc = unit_cost<R, ST, NT, D>(v, v->order[first + q], um.x, um.y, um.z, RefStats{os.x, os.y},
+                                                     s_win + o * Win<R, ST>::VEC, s_ref, tw, olx, oly, x0 + olx, oy,
+                                                     sc.soft_mask);
+                    *sm.unit(first + q, k) = uc;
+                }
+                __syncthreads();  // the part's source costs are complete
+                if (last == S) break;
+                // The kk-th lowest of all source costs is at least the lowest of the leading S - kk + 1, so the
+                // mean is at least that over kk (rounded addition and division are monotone): a trial whose bound
+                // reaches the pixel's cost cannot win, and the remaining sources are sampled for the others only.
+                float low = 2.0f;
+                for (int q = 0; q < lead; ++q) low = fminf(low, *sm.unit(q, tid));
+                keep = active && (!sc.memo || __fdiv_rn(low, static_cast<float>(kk)) < best_cost);
+                const unsigned votes = __ballot_sync(0xffffffffu, keep);
+                int at = 0;
+                if (lane == 0 && votes) at = atomicAdd(&sm.survivors, __popc(votes));
+                at = __shfl_sync(0xffffffffu, at, 0);
+                if (keep) sm.items[at + __popc(votes & ((1u << lane) - 1u))] = static_cast<unsigned short>(tid);
+                __syncthreads();  // the survivors' list is complete
+                units = sm.survivors;
+                first = lead;
+                last = S;
             }
-            __syncthreads();  // the chunk's source costs are complete
-            if (tid < n) {
+            if (tid < n && keep) {
                 Lowest low;
                 for (int s = 0; s < S; ++s) low.insert(*sm.unit(s, tid));
-                c = low.mean(min(sc.top_k, S));
+                c = low.mean(kk);
                 if (round == 0) sm.cost[item] = c;
             }
         }
@@ -789,7 +817,7 @@ __device__ __forceinline__ void tile_propagate16(const ViewDesc* v, int tile_x, 
                     }
                 }
             }
-        } else if (active && c < best_cost) {
+        } else if (active && keep && c < best_cost) {
             best_cost = c;
             settled = false;
             best = trial;

@@ -35,6 +35,7 @@ struct ViewDesc {
     float* cost;                      // H*W; sign bit: see cost_settled (hp_tile.cuh)
     int ref_pitch, ref16_pitch;
     int W, H, S;
+    unsigned char order[HP_MAX_SOURCES];  // sources by descending baseline (order_sources)
     int tiles_x, tiles_y;
     int tile_h;                       // rows of a tile (a CTA has tile_h warps, one per row)
     float dmin, dmax;
@@ -55,6 +56,20 @@ struct ViewDesc {
     const int* seed_map;
     const hp_seed* seeds;
 };
+
+// Fills v->order from the coefficients: sources by the image-plane length of
+// b = K_s t_rel, longest first (ties: lower index first).  Only the order in
+// which a half-pass samples sources depends on it, never a result.
+inline void order_sources(ViewDesc* v) {
+    float len[HP_MAX_SOURCES];
+    for (int s = 0; s < v->S; ++s) {
+        const float l = v->ab[s][9] * v->ab[s][9] + v->ab[s][10] * v->ab[s][10];
+        int k = s;
+        for (; k > 0 && len[v->order[k - 1]] < l; --k) v->order[k] = v->order[k - 1];
+        v->order[k] = static_cast<unsigned char>(s);
+        len[s] = l;
+    }
+}
 
 // Solver constants for one launch.
 // SolveConsts::soft_mask bit 31 (tests only): no corner-test shortcuts in the

@@ -153,6 +153,7 @@ extern "C" hp_status hp_solve_static(int device, void* stream, const hp_job* job
         for (int s = 0; s < job->num_sources; ++s)
             for (int i = 0; i < 12; ++i) d.ab[s][i] = static_cast<float>(ab[12 * s + i]);
     }
+    hp::order_sources(&d);
     d.tile_h = hp::TILE_H;
     d.tiles_x = (width + hp::TILE_W - 1) / hp::TILE_W;
     d.tiles_y = (height + hp::TILE_H - 1) / hp::TILE_H;
