@@ -34,6 +34,7 @@
 #include "hp_internal.h"
 #include "hp_rng.cuh"
 #include "hp_filter.cuh"
+#include "hp_pass.cuh"
 #include "hp_tile.cuh"
 
 #ifndef HP_F16_MIN_BLOCKS
@@ -117,13 +118,9 @@ struct alignas(16) Shared {
     float4 plane[NT];               // half-pass: plane_vector of the chunk's items
     float ref[OVERLAY ? (REF > UNITS ? REF : UNITS) : REF];
     float unit_own[OVERLAY ? 1 : UNITS];
-    float cost[NT * 4];             // half-pass: neighbour costs, slot (thread << 2 | cand)
     float2 stat[NT];                // half-pass: (mean, ssd) of each thread's pixel window
-    unsigned short items[NT * 4];   // half-pass: CTA item list, thread << 2 | cand
-    int warp_total[TH];
-    int survivors;                  // half-pass: entries of the refinement round's second list
-    // Half-pass: cost of the chunk's item k at source s.
-    __device__ __forceinline__ float* unit(int s, int k) { return (OVERLAY ? ref : unit_own) + s * NT + k; }
+    PassShared<NT> pass;
+    __device__ __forceinline__ float* units() { return OVERLAY ? ref : unit_own; }  // half-pass: source costs
 };
 
 template <int R, int ST, int NT>
@@ -580,26 +577,6 @@ __device__ __forceinline__ float unit_cost(const ViewDesc* __restrict__ v, int s
     return c;
 }
 
-// Mean of the min(topk, S) lowest source costs, inserted one by one.
-struct Lowest {
-    float top0 = 2.0f, top1 = 2.0f, top2 = 2.0f;
-    __device__ __forceinline__ void insert(float c) {
-        if (c < top2) {
-            top2 = c;
-            if (top2 < top1) {
-                float t = top1; top1 = top2; top2 = t;
-                if (top1 < top0) { t = top0; top0 = top1; top1 = t; }
-            }
-        }
-    }
-    __device__ __forceinline__ float mean(int kk) const {
-        float sum = top0;
-        if (kk > 1) sum = __fadd_rn(sum, top1);
-        if (kk > 2) sum = __fadd_rn(sum, top2);
-        return __fdiv_rn(sum, static_cast<float>(kk));
-    }
-};
-
 extern __shared__ __align__(16) unsigned char dynamic_smem[];
 template <int R, int ST, int TH>
 __device__ __forceinline__ Shared<R, ST, TH>& shared_of() {
@@ -633,7 +610,8 @@ __device__ __forceinline__ void tile_cost16(const ViewDesc* v, int tile_x, int t
                 low.insert(unit_cost<R, ST, NT, D>(v, s, m.x, m.y, m.z, st,
                                                    s_win + threadIdx.x * Win<R, ST>::VEC, s_ref, tw, lx, ly, x, y,
                                                    sc.soft_mask));
-        v->cost[idx] = low.mean(min(sc.top_k, v->S));
+        const int kk = min(sc.top_k, v->S);
+        v->cost[idx] = __fdiv_rn(low.sum(kk), static_cast<float>(kk));
     }
 }
 
@@ -644,188 +622,40 @@ __global__ void __launch_bounds__(Tile<TH>::NT, Tile<TH>::MIN_BLOCKS) cost16_ker
     tile_cost16<R, ST, TH, D>(v, tile_x, tile_y, sc, shared_of<R, ST, TH>());
 }
 
-// One red-black half-pass.  Scoring is split into units of (item, source): an
-// item is a pixel with a plane to score, and the CTA's threads take the units
-// of up to NT items in order (unit u: item u % n, source u / n), so every warp
-// has full lanes whatever the number of items and whatever sources each warp
-// would have drawn.  Scored in rounds: the neighbour planes of all pixels of
-// the tile (every lane lists the ones its pixel must score, the lists of all
-// warps concatenated), then one round per refinement step with one perturbed
-// plane per pixel.  A unit reads its pixel's window statistics and s_win
-// column from shared memory; owners fold their costs in L, R, U, D order
-// exactly as if they had scored them themselves, so results do not depend on
-// which lane scored what.
+// Scorer of the half-pass (red_black_pass): a unit reads its pixel's window
+// statistics and s_win column, and its item's plane vector, from shared memory.
+template <int R, int ST, int TH, int D>
+struct Scorer16 {
+    static constexpr int NT = Tile<TH>::NT, TW = TILE_W + 2 * R;
+    const ViewDesc* v;
+    Shared<R, ST, TH>& sm;
+    int x0, y0;
+    unsigned soft_mask;
+    RefStats st{0.f, 0.f};
+    __device__ __forceinline__ void begin(int lx, int ly) { st = load_window<R, ST, NT>(sm.win, sm.ref, TW, lx, ly); }
+    __device__ __forceinline__ void publish() { sm.stat[threadIdx.x] = make_float2(st.mean, st.ssd); }
+    __device__ __forceinline__ void set_plane(int k, int x, int y, float4 h, bool ok) {
+        sm.plane[k] = ok ? plane_vector(v, x, y, h) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    __device__ __forceinline__ float score(int s, int k, int o, int lx, int ly) const {
+        const float2 os = sm.stat[o];
+        const float4 m = sm.plane[k];
+        if (m.w == 0.0f) return 2.0f;
+        return unit_cost<R, ST, NT, D>(v, s, m.x, m.y, m.z, RefStats{os.x, os.y}, sm.win + o * Win<R, ST>::VEC,
+                                       sm.ref, TW, lx, ly, x0 + lx, y0 + ly, soft_mask);
+    }
+    __device__ __forceinline__ float mean(float sum, int k) const { return __fdiv_rn(sum, static_cast<float>(k)); }
+};
+
 template <int R, int ST, int TH, int D>
 __device__ __forceinline__ void tile_propagate16(const ViewDesc* v, int tile_x, int tile_y, const SolveConsts& sc,
                                                  int iteration, int color, Shared<R, ST, TH>& sm) {
-    constexpr int NT = Tile<TH>::NT, WARPS = TH;
-    float* s_ref = sm.ref;
-    __half2* s_win = sm.win;
-    constexpr int tw = TILE_W + 2 * R, th = TH + 2 * R;
+    constexpr int NT = Tile<TH>::NT;
     const int x0 = tile_x * TILE_W, y0 = tile_y * TH;
-    load_ref_tile16<NT>(s_ref, tw, th, v, x0, y0, R);
+    load_ref_tile16<NT>(sm.ref, TILE_W + 2 * R, TH + 2 * R, v, x0, y0, R);
     __syncthreads();
-    const int W = v->W, H = v->H, S = v->S;
-    const int tid = threadIdx.x, ly = tid >> 5, lane = tid & 31;
-    const int y = y0 + ly;
-    const int lx = 2 * lane + ((y + color) & 1);
-    const int x = x0 + lx;
-    const bool active = y < H && x < W;  // every thread takes part in the CTA barriers below
-    const size_t idx = static_cast<size_t>(y) * W + x;
-    RefStats st{0.f, 0.f};
-    float4 best = make_float4(0.f, 0.f, 0.f, 0.f);
-    float best_cost = 0.f;
-    unsigned need = 0;
-    bool settled = true;
-    if (active) {
-        st = load_window<R, ST, NT>(s_win, s_ref, tw, lx, ly);
-        best = v->hyp[idx];
-        best_cost = cost_value(v->cost[idx]);
-        need = neighbour_needs(v, x, y, best, sc.memo && iteration > 0);
-    }
-    sm.stat[tid] = make_float2(st.mean, st.ssd);
-    const int cnt = __popc(need);
-    int incl = cnt;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int t = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += t;
-    }
-    if (lane == 31) sm.warp_total[ly] = incl;
-    __syncthreads();  // warp totals, window statistics and s_win columns are complete
-    int total = 0;
-    {
-        int k = incl - cnt;
-#pragma unroll
-        for (int w = 0; w < WARPS; ++w) {
-            const int t = sm.warp_total[w];
-            k += w < ly ? t : 0;
-            total += t;
-        }
-        for (int cand = 0; cand < 4; ++cand)
-            if (need & (1u << cand)) sm.items[k++] = static_cast<unsigned short>((tid << 2) | cand);
-    }
-    __syncthreads();  // the CTA's item list is complete
-    const int kk = min(sc.top_k, S), lead = S - kk + 1;
-    float drange = __fmul_rn(__fsub_rn(v->dmax, v->dmin), 0.5f);
-    float nrange = 1.0f;
-    for (int i = 0; i < iteration; ++i) {
-        drange = __fmul_rn(drange, sc.iter_decay);
-        nrange = __fmul_rn(nrange, sc.iter_decay);
-    }
-#pragma unroll 1
-    for (int round = 0; round <= sc.refine_steps; ++round) {
-        float4 trial = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (round > 0) {
-            if (active) {
-                const uint4 rr =
-                    philox4x32_10(make_uint4(static_cast<uint32_t>(idx), v->view_id,
-                                             1u + static_cast<uint32_t>(iteration), static_cast<uint32_t>(round - 1)),
-                                  v->seed_lo, v->seed_hi);
-                const float cd = __fmaf_rn(__fmaf_rn(u01(rr.x), 2.0f, -1.0f), drange, best.x);
-                const float cx = __fmaf_rn(__fmaf_rn(u01(rr.y), 2.0f, -1.0f), nrange, best.y);
-                const float cy = __fmaf_rn(__fmaf_rn(u01(rr.z), 2.0f, -1.0f), nrange, best.z);
-                const float cz = __fmaf_rn(__fmaf_rn(u01(rr.w), 2.0f, -1.0f), nrange, best.w);
-                float3 cn = normalize3_rn(cx, cy, cz);
-                if (dot3_rn(cn, view_ray(v->kinv, x, y)) > 0.0f) cn = make_float3(-cn.x, -cn.y, -cn.z);
-                trial = make_float4(fmaxf(v->dmin, fminf(v->dmax, cd)), cn.x, cn.y, cn.z);
-            }
-            drange = __fmul_rn(drange, sc.step_decay);
-            nrange = __fmul_rn(nrange, sc.step_decay);
-        }
-        const int count = round == 0 ? total : NT;
-        float c = 2.0f;
-        bool keep = true;
-#pragma unroll 1
-        for (int c0 = 0; c0 < count; c0 += NT) {
-            const int n = min(NT, count - c0);
-            int item = tid << 2;
-            float4 m = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (round > 0) {
-                if (active) m = plane_vector(v, x, y, trial);
-            } else if (tid < n) {
-                item = sm.items[c0 + tid];
-                const int o = item >> 2, cand = item & 3;
-                const int oy = y0 + (o >> 5), ox = x0 + 2 * (o & 31) + ((oy + color) & 1);
-                const int nxp = ox + (cand == 0 ? -1 : (cand == 1 ? 1 : 0));
-                const int nyp = oy + (cand == 2 ? -1 : (cand == 3 ? 1 : 0));
-                if (HP_CHECK(nxp >= 0 && nxp < W && nyp >= 0 && nyp < H, HP_CHECK_NEIGHBOUR, ox, oy, nxp, nyp, W, H,
-                             0.f, 0.f, 0.f, 0.f))
-                    m = plane_vector(v, ox, oy, v->hyp[static_cast<size_t>(nyp) * W + nxp]);
-            }
-            sm.plane[tid] = m;
-            if (tid == 0) sm.survivors = 0;
-            __syncthreads();  // the chunk's planes are complete
-            // Sources first .. last - 1 of the view's order, for the chunk's items (a refinement round's second
-            // part: for the listed survivors).
-            int units = n, first = 0, last = round == 0 ? S : lead;
-#pragma unroll 1
-            for (;;) {
-#pragma unroll 1
-                for (int u = tid; u < units * (last - first); u += NT) {
-                    const int q = u / units;
-                    int k = u - q * units;
-                    if (first > 0) k = sm.items[k];
-                    const int o = round == 0 ? sm.items[c0 + k] >> 2 : k;
-                    const int oly = o >> 5, oy = y0 + oly, olx = 2 * (o & 31) + ((oy + color) & 1);
-                    const float2 os = sm.stat[o];
-                    const float4 um = sm.plane[k];
-                    float uc = 2.0f;
-                    if (um.w != 0.0f)
-                        uc = unit_cost<R, ST, NT, D>(v, v->order[first + q], um.x, um.y, um.z, RefStats{os.x, os.y},
-                                                     s_win + o * Win<R, ST>::VEC, s_ref, tw, olx, oly, x0 + olx, oy,
-                                                     sc.soft_mask);
-                    *sm.unit(first + q, k) = uc;
-                }
-                __syncthreads();  // the part's source costs are complete
-                if (last == S) break;
-                // The kk-th lowest of all source costs is at least the lowest of the leading S - kk + 1, so the
-                // mean is at least that over kk (rounded addition and division are monotone): a trial whose bound
-                // reaches the pixel's cost cannot win, and the remaining sources are sampled for the others only.
-                float low = 2.0f;
-                for (int q = 0; q < lead; ++q) low = fminf(low, *sm.unit(q, tid));
-                keep = active && (!sc.memo || __fdiv_rn(low, static_cast<float>(kk)) < best_cost);
-                const unsigned votes = __ballot_sync(0xffffffffu, keep);
-                int at = 0;
-                if (lane == 0 && votes) at = atomicAdd(&sm.survivors, __popc(votes));
-                at = __shfl_sync(0xffffffffu, at, 0);
-                if (keep) sm.items[at + __popc(votes & ((1u << lane) - 1u))] = static_cast<unsigned short>(tid);
-                __syncthreads();  // the survivors' list is complete
-                units = sm.survivors;
-                first = lead;
-                last = S;
-            }
-            if (tid < n && keep) {
-                Lowest low;
-                for (int s = 0; s < S; ++s) low.insert(*sm.unit(s, tid));
-                c = low.mean(kk);
-                if (round == 0) sm.cost[item] = c;
-            }
-        }
-        if (round == 0) {
-            __syncthreads();  // every neighbour cost is in its owner's slot
-#pragma unroll
-            for (int cand = 0; cand < 4; ++cand) {
-                if (need & (1u << cand)) {
-                    const float nc = sm.cost[(tid << 2) | cand];
-                    if (nc < best_cost) {
-                        const int nxp = x + (cand == 0 ? -1 : (cand == 1 ? 1 : 0));
-                        const int nyp = y + (cand == 2 ? -1 : (cand == 3 ? 1 : 0));
-                        best_cost = nc;
-                        settled = false;
-                        best = v->hyp[static_cast<size_t>(nyp) * W + nxp];
-                    }
-                }
-            }
-        } else if (active && keep && c < best_cost) {
-            best_cost = c;
-            settled = false;
-            best = trial;
-        }
-    }
-    if (!active) return;
-    v->hyp[idx] = best;
-    v->cost[idx] = sc.memo && settled ? -best_cost : best_cost;
+    Scorer16<R, ST, TH, D> scorer{v, sm, x0, y0, sc.soft_mask};
+    red_black_pass<NT>(v, x0, y0, sc, iteration, color, scorer, sm.units(), sm.pass);
 }
 
 template <int R, int ST, int TH, int D>

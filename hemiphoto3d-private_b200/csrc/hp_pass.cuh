@@ -1,0 +1,243 @@
+// The red-black half-pass of one tile (propagate_and_refine_kernel,
+// src/dense_recon/patchmatch_mvs.cu:519-655), shared by the FP32 and FP16
+// kernels: which planes are scored, by which lanes, and how a pixel adopts one.
+// A scorer supplies the arithmetic of a cost.
+//
+// Scoring is split into units of (item, source): an item is a pixel with a
+// plane to score, and the CTA's threads take the units of up to NT items in
+// order (unit u: item u % n, source u / n).  Every warp then has full lanes
+// whatever the number of items, where one lane per item, all sources in a row,
+// left the last warps of a list of ~390 items idle for six sources at a time.
+// Rounds: the neighbour planes of all pixels of the tile (L, R, U, D; every
+// lane lists the ones its pixel must score, the lists concatenated), then one
+// round per refinement step with one perturbed plane per pixel.  Owners fold
+// their costs in L, R, U, D order with a strict less, exactly as if they had
+// scored them one after the other, so results depend neither on which lane
+// scored what nor on the tile's shape.
+//
+// A refinement trial is rarely better than the plane it perturbs, and usually
+// much worse: on 1920 x 1080, r 7, s 2, 6 sources, 80-95% of the trials of
+// iterations 1 to 7 are beaten by the bound below after 4 of 6 sources, 35%
+// still in iteration 11.  So its sources are sampled in two parts, longest
+// baseline first (there a wrong plane shows most): all trials on the leading
+// S - k + 1 sources, k = min(top_k, S), and on the others only the trials that
+// can still win.  Neighbour planes mostly win or come close, so theirs are
+// sampled in one part.  Measured with the settled-neighbour rule
+// (neighbour_needs), before -> after: FP16-acc 4 x 1920 x 1080, r 7, s 2, 6
+// sources, 12 iterations 143.3 -> 126.9 ms; 3000 x 2000, 8 sources 132.9 ->
+// 117.2 ms; r 5, s 1 on 1920 x 1080 65.9 -> 56.1 ms.
+#pragma once
+
+#include "hp_check.cuh"
+#include "hp_internal.h"
+#include "hp_rng.cuh"
+#include "hp_tile.cuh"
+
+namespace hp {
+
+// The three lowest source costs, inserted one by one.  A cost of 2 (the worst)
+// changes nothing, so sources without a valid window need not be inserted.
+struct Lowest {
+    float top0 = 2.0f, top1 = 2.0f, top2 = 2.0f;
+    __device__ __forceinline__ void insert(float c) {
+        if (c < top2) {
+            top2 = c;
+            if (top2 < top1) {
+                float t = top1; top1 = top2; top2 = t;
+                if (top1 < top0) { t = top0; top0 = top1; top1 = t; }
+            }
+        }
+    }
+    __device__ __forceinline__ float sum(int k) const {
+        float s = top0;
+        if (k > 1) s = __fadd_rn(s, top1);
+        if (k > 2) s = __fadd_rn(s, top2);
+        return s;
+    }
+};
+
+// Shared memory of a half-pass with NT threads, beyond the scorer's own and the
+// source costs (HP_MAX_SOURCES rows of NT floats: cost of item k at the q-th
+// source of the view's order at q * NT + k).
+template <int NT>
+struct PassShared {
+    float cost[NT * 4];            // neighbour costs, slot (thread << 2 | cand)
+    unsigned short items[NT * 4];  // neighbour items (thread << 2 | cand), then the surviving trials
+    int warp_total[NT / 32];
+    int survivors;
+};
+
+// One half-pass of the tile at (x0, y0): TILE_W x NT / 32 pixels, thread
+// (row, lane) owns pixel x0 + 2 * lane + ((y + color) & 1) of row y0 + row, so
+// every thread has work, where the reference idles half its grid.
+// The scorer K, per thread:
+//   begin(lx, ly)               prepares the window of the thread's own pixel (active pixels only)
+//   publish()                   makes it readable by the other threads (after the next barrier)
+//   set_plane(k, x, y, h, ok)   thread k: plane h of item k at pixel (x, y), ok false: no plane
+//   score(source, k, o, lx, ly) cost of item k, whose pixel is thread o's, at tile position (lx, ly)
+//   mean(sum, k)                sum / k, monotone in sum
+template <int NT, class K>
+__device__ __forceinline__ void red_black_pass(const ViewDesc* v, int x0, int y0, const SolveConsts& sc,
+                                               int iteration, int color, K& scorer, float* unit,
+                                               PassShared<NT>& sm) {
+    const int W = v->W, H = v->H, S = v->S;
+    const int tid = threadIdx.x, ly = tid >> 5, lane = tid & 31;
+    const int y = y0 + ly;
+    const int lx = 2 * lane + ((y + color) & 1);
+    const int x = x0 + lx;
+    const bool active = y < H && x < W;  // every thread takes part in the barriers
+    const size_t idx = static_cast<size_t>(y) * W + x;
+    float4 best = make_float4(0.f, 0.f, 0.f, 0.f);
+    float best_cost = 0.f;
+    unsigned need = 0;
+    bool settled = true;
+    if (active) {
+        scorer.begin(lx, ly);
+        best = v->hyp[idx];
+        best_cost = cost_value(v->cost[idx]);
+        need = neighbour_needs(v, x, y, best, sc.memo && iteration > 0);
+    }
+    scorer.publish();
+    // Exclusive scan of the item counts over the warp, then over the CTA's warps.
+    const int cnt = __popc(need);
+    int incl = cnt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += t;
+    }
+    if (lane == 31) sm.warp_total[ly] = incl;
+    __syncthreads();
+    int total = 0;
+    {
+        int k = incl - cnt;
+#pragma unroll
+        for (int w = 0; w < NT / 32; ++w) {
+            const int t = sm.warp_total[w];
+            k += w < ly ? t : 0;
+            total += t;
+        }
+        for (int cand = 0; cand < 4; ++cand)
+            if (need & (1u << cand)) sm.items[k++] = static_cast<unsigned short>((tid << 2) | cand);
+    }
+    __syncthreads();  // the item list is complete
+    const int kk = min(sc.top_k, S), lead = S - kk + 1;
+    float drange = __fmul_rn(__fsub_rn(v->dmax, v->dmin), 0.5f);
+    float nrange = 1.0f;
+    for (int i = 0; i < iteration; ++i) {
+        drange = __fmul_rn(drange, sc.iter_decay);
+        nrange = __fmul_rn(nrange, sc.iter_decay);
+    }
+#pragma unroll 1
+    for (int round = 0; round <= sc.refine_steps; ++round) {
+        float4 trial = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (round > 0) {
+            // Random refinement around the running best (:583-648).
+            if (active) {
+                const uint4 rr =
+                    philox4x32_10(make_uint4(static_cast<uint32_t>(idx), v->view_id,
+                                             1u + static_cast<uint32_t>(iteration), static_cast<uint32_t>(round - 1)),
+                                  v->seed_lo, v->seed_hi);
+                const float cd = __fmaf_rn(__fmaf_rn(u01(rr.x), 2.0f, -1.0f), drange, best.x);
+                const float cx = __fmaf_rn(__fmaf_rn(u01(rr.y), 2.0f, -1.0f), nrange, best.y);
+                const float cy = __fmaf_rn(__fmaf_rn(u01(rr.z), 2.0f, -1.0f), nrange, best.z);
+                const float cz = __fmaf_rn(__fmaf_rn(u01(rr.w), 2.0f, -1.0f), nrange, best.w);
+                float3 cn = normalize3_rn(cx, cy, cz);
+                if (dot3_rn(cn, view_ray(v->kinv, x, y)) > 0.0f) cn = make_float3(-cn.x, -cn.y, -cn.z);
+                trial = make_float4(fmaxf(v->dmin, fminf(v->dmax, cd)), cn.x, cn.y, cn.z);
+            }
+            drange = __fmul_rn(drange, sc.step_decay);
+            nrange = __fmul_rn(nrange, sc.step_decay);
+        }
+        const int count = round == 0 ? total : NT;
+        float c = 2.0f;
+        bool keep = true;
+#pragma unroll 1
+        for (int c0 = 0; c0 < count; c0 += NT) {
+            const int n = min(NT, count - c0);
+            int item = tid << 2;
+            if (round > 0) {
+                scorer.set_plane(tid, x, y, trial, active);
+            } else if (tid < n) {
+                item = sm.items[c0 + tid];
+                const int o = item >> 2, cand = item & 3;
+                const int oy = y0 + (o >> 5), ox = x0 + 2 * (o & 31) + ((oy + color) & 1);
+                const int nxp = ox + (cand == 0 ? -1 : (cand == 1 ? 1 : 0));
+                const int nyp = oy + (cand == 2 ? -1 : (cand == 3 ? 1 : 0));
+                float4 h = make_float4(0.f, 0.f, 0.f, 0.f);
+                const bool ok = HP_CHECK(nxp >= 0 && nxp < W && nyp >= 0 && nyp < H, HP_CHECK_NEIGHBOUR, ox, oy, nxp,
+                                         nyp, W, H, 0.f, 0.f, 0.f, 0.f);
+                if (ok) h = v->hyp[static_cast<size_t>(nyp) * W + nxp];
+                scorer.set_plane(tid, ox, oy, h, ok);
+            }
+            if (tid == 0) sm.survivors = 0;
+            __syncthreads();  // the chunk's planes are complete
+            // Sources first .. last - 1 of the view's order, for the chunk's items (second part: the listed ones).
+            int units = n, first = 0, last = round == 0 ? S : lead;
+#pragma unroll 1
+            for (;;) {
+#pragma unroll 1
+                for (int q = first; q < last; ++q) {
+                    const int source = v->order[q];
+                    // The first warp to take a batch of this source follows the one that took the previous source's last.
+                    const int turn = (q - first) * ((units + 31) >> 5);
+#pragma unroll 1
+                    for (int u = ((ly - turn) & (NT / 32 - 1)) * 32 + lane; u < units; u += NT) {
+                        const int k = first > 0 ? sm.items[u] : u;
+                        const int o = round == 0 ? sm.items[c0 + k] >> 2 : k;
+                        const int oly = o >> 5;
+                        unit[q * NT + k] = scorer.score(source, k, o, 2 * (o & 31) + ((y0 + oly + color) & 1), oly);
+                    }
+                }
+                __syncthreads();  // the part's source costs are complete
+                if (last == S) break;
+                // The k-th lowest of all source costs is at least the lowest of the leading S - k + 1, so the mean is
+                // at least that over k (rounded addition and mean() are monotone): a trial whose bound reaches the
+                // pixel's cost cannot win.  A half-pass on caller maps (memo off) samples every trial whole.
+                float low = 2.0f;
+                for (int q = 0; q < lead; ++q) low = fminf(low, unit[q * NT + tid]);
+                keep = active && (!sc.memo || scorer.mean(low, kk) < best_cost);
+                const unsigned votes = __ballot_sync(0xffffffffu, keep);
+                int at = 0;
+                if (lane == 0 && votes) at = atomicAdd(&sm.survivors, __popc(votes));
+                at = __shfl_sync(0xffffffffu, at, 0);
+                if (keep) sm.items[at + __popc(votes & ((1u << lane) - 1u))] = static_cast<unsigned short>(tid);
+                __syncthreads();  // the survivors' list is complete
+                units = sm.survivors;
+                first = lead;
+                last = S;
+            }
+            if (tid < n && keep) {
+                Lowest low;
+                for (int q = 0; q < S; ++q) low.insert(unit[q * NT + tid]);
+                c = scorer.mean(low.sum(kk), kk);
+                if (round == 0) sm.cost[item] = c;
+            }
+        }
+        if (round == 0) {
+            __syncthreads();  // every neighbour cost is in its owner's slot
+#pragma unroll
+            for (int cand = 0; cand < 4; ++cand) {
+                if (need & (1u << cand)) {
+                    const float nc = sm.cost[(tid << 2) | cand];
+                    if (nc < best_cost) {
+                        const int nxp = x + (cand == 0 ? -1 : (cand == 1 ? 1 : 0));
+                        const int nyp = y + (cand == 2 ? -1 : (cand == 3 ? 1 : 0));
+                        best_cost = nc;
+                        settled = false;
+                        best = v->hyp[static_cast<size_t>(nyp) * W + nxp];
+                    }
+                }
+            }
+        } else if (active && keep && c < best_cost) {
+            best_cost = c;
+            settled = false;
+            best = trial;
+        }
+    }
+    if (!active) return;
+    v->hyp[idx] = best;
+    v->cost[idx] = sc.memo && settled ? -best_cost : best_cost;
+}
+
+}  // namespace hp
