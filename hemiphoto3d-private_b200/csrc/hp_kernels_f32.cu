@@ -26,7 +26,7 @@
 
 // Resident CTAs per SM the cost kernels are register-budgeted for.
 #ifndef HP_F32_MIN_BLOCKS
-#define HP_F32_MIN_BLOCKS 2
+#define HP_F32_MIN_BLOCKS 3
 #endif
 
 namespace hp {
@@ -99,6 +99,23 @@ __device__ __forceinline__ float rcp_approx(float x) {
 // row-invariant products a1*y are computed once per row (the same rounded
 // value), and samples are accumulated in tap order, skipping invalid taps
 // exactly as the reference's `continue`s do.
+// Sums of the reference window and of its squares in tap order: what the taps
+// of any source add up to when all of them are valid.
+template <int R, int ST>
+__device__ __forceinline__ float2 window_sums(const float* __restrict__ s_ref, int tw, int lx, int ly) {
+    constexpr int SIDE = (2 * R) / ST + 1;
+    float sum = 0.0f, sum2 = 0.0f;
+#pragma unroll 1
+    for (int i = 0; i < SIDE; ++i)
+#pragma unroll
+        for (int j = 0; j < SIDE; ++j) {
+            const float rv = s_ref[(ly + i * ST) * tw + lx + j * ST];
+            sum = __fadd_rn(sum, rv);
+            sum2 = __fmaf_rn(rv, rv, sum2);
+        }
+    return make_float2(sum, sum2);
+}
+
 struct PlaneF32 {
     float nK0, nK1, nK2;  // K^-T n
     float inv_n_dot_P;
@@ -130,10 +147,12 @@ __device__ __forceinline__ PlaneF32 plane_f32(const ViewDesc* __restrict__ v, in
 // Cost of source s under the plane p at pixel (x, y), tile position (lx, ly).
 template <int R, int ST>
 __device__ __forceinline__ float cost_f32(const float* __restrict__ s_ref, int tw, int lx, int ly, int x, int y,
-                                          const PlaneF32& p, const ViewDesc* __restrict__ v, int s) {
+                                          const PlaneF32& p, float2 ref_sums, const ViewDesc* __restrict__ v,
+                                          int s) {
+    constexpr unsigned WARP = 0xffffffffu;
     constexpr int SIDE = (2 * R) / ST + 1;
     constexpr int min_count = (SIDE * SIDE) / 2;
-    const float nK0 = p.nK0, nK1 = p.nK1, nK2 = p.nK2, inv_n_dot_P = p.inv_n_dot_P;
+    const float nK0 = p.nK0, nK1 = p.nK1, nK2 = p.nK2, inv_n_dot_P = p.ok ? p.inv_n_dot_P : 0.0f;
     const float fx = static_cast<float>(x);
     const float fy = static_cast<float>(y);
     const float fw1 = static_cast<float>(v->W) - 1.0f;
@@ -144,19 +163,25 @@ __device__ __forceinline__ float cost_f32(const float* __restrict__ s_ref, int t
     const cudaTextureObject_t tex = v->src_tex[s];
     float sum_ref = 0.0f, sum_src = 0.0f, sum_ref2 = 0.0f, sum_src2 = 0.0f, sum_rs = 0.0f;
     int count = 0;
-    // A window whose warp lies wholly beyond one edge of the source has no
-    // valid tap, so the reference's count rule gives 2 for this source:
-    // skip its taps.  The test runs on the plane-induced homography
-    // H = A + b (K^-T n)^T / (n.P) at the window's corners, in front of
-    // the camera (w_z > 1e-6, so the warped window is the convex quad of
-    // its corners) and past the edge by 0.25 px, far above the rounding
-    // differences between this and the per-tap arithmetic below.
+    // Two decisions from the window's corners under the plane-induced
+    // homography H = A + b (K^-T n)^T / (n.P); in front of the camera
+    // (w_z > 1e-6) the warped window is the convex quad of its corners.
+    // Wholly beyond one edge of the source by 0.25 px: no valid tap, so the
+    // reference's count rule gives 2 and no tap is sampled.  Wholly inside by
+    // 0.25 px: every tap is valid, and needs no test of its own.  The margin
+    // covers the rounding differences between this and the per-tap arithmetic
+    // below for the second decision while 16 roundings of the largest partial
+    // sums of either (Mx = |A| and |b| |m| terms over the window, likewise My,
+    // Mz), at most (Mx + |u| Mz) 2^-20 / w_z, stay under 0.2 px; |u| and |v|
+    // are below the image's sides there.
+    bool inside, sampled = p.ok;
     {
         const float m0 = nK0 * inv_n_dot_P, m1 = nK1 * inv_n_dot_P, m2 = nK2 * inv_n_dot_P;
         const float hz0 = fmaf(b2, m0, a6), hz1 = fmaf(b2, m1, a7), hz2 = fmaf(b2, m2, a8);
         const float hx0 = fmaf(b0, m0, a0), hx1 = fmaf(b0, m1, a1), hx2 = fmaf(b0, m2, a2);
         const float hy0 = fmaf(b1, m0, a3), hy1 = fmaf(b1, m1, a4), hy2 = fmaf(b1, m2, a5);
-        bool front = true, left = true, right = true, top_ = true, bottom = true;
+        bool left = true, right = true, top_ = true, bottom = true;
+        float in = 1e30f, zmin = 1e30f;
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
             const float px = fx + static_cast<float>((c & 1) ? (SIDE - 1) * ST - R : -R);
@@ -164,52 +189,101 @@ __device__ __forceinline__ float cost_f32(const float* __restrict__ s_ref, int t
             const float wz = fmaf(hz0, px, fmaf(hz1, py, hz2));
             const float wx = fmaf(hx0, px, fmaf(hx1, py, hx2));
             const float wy = fmaf(hy0, px, fmaf(hy1, py, hy2));
-            front = front && wz > 1e-6f;
+            zmin = fminf(zmin, wz);
             left = left && wx < -0.25f * wz;
             right = right && wx >= (fw1 + 0.25f) * wz;
             top_ = top_ && wy < -0.25f * wz;
             bottom = bottom && wy >= (fh1 + 0.25f) * wz;
+            in = fminf(in, fminf(fminf(fmaf(-0.25f, wz, wx), fmaf(fw1 - 0.25f, wz, -wx)),
+                                 fminf(fmaf(-0.25f, wz, wy), fmaf(fh1 - 0.25f, wz, -wy))));
         }
-        if (front && (left || right || top_ || bottom)) return 2.0f;
+        const bool front = zmin > 1e-6f;
+        if (front && (left || right || top_ || bottom)) sampled = false;
+        const float X = fabsf(fx) + static_cast<float>(SIDE * ST), Y = fabsf(fy) + static_cast<float>(SIDE * ST);
+        const float Ms = fmaf(fabsf(m0), X, fmaf(fabsf(m1), Y, fabsf(m2)));
+        const float Mx = fmaf(fabsf(b0), Ms, fmaf(fabsf(a0), X, fmaf(fabsf(a1), Y, fabsf(a2))));
+        const float My = fmaf(fabsf(b1), Ms, fmaf(fabsf(a3), X, fmaf(fabsf(a4), Y, fabsf(a5))));
+        const float Mz = fmaf(fabsf(b2), Ms, fmaf(fabsf(a6), X, fmaf(fabsf(a7), Y, fabsf(a8))));
+        // Not-a-numbers fail: `in` ignores them, the bound does not.
+        inside = front && in > 0.0f && fmaf(fw1, Mz, Mx) <= 2e5f * zmin && fmaf(fh1, Mz, My) <= 2e5f * zmin;
     }
 #ifdef HP_COUNT_TAPS
     atomicAdd(&g_taps32, static_cast<unsigned long long>(SIDE * SIDE));
 #endif
+    if (!__any_sync(WARP, sampled)) return 2.0f;
+    if (__all_sync(WARP, inside || !sampled)) {
+        // Every tap of every sampled lane is valid: no tests, and the reference
+        // sums are the window's own.  The same operations on the same values
+        // as below, so the same bits.
+        sum_ref = ref_sums.x;
+        sum_ref2 = ref_sums.y;
+        count = SIDE * SIDE;
 #pragma unroll 1
-    for (int i = 0; i < SIDE; ++i) {
-        const float wpy = fy + static_cast<float>(i * ST - R);
-        const float tqx = __fmul_rn(a1, wpy), tqy = __fmul_rn(a4, wpy), tqz = __fmul_rn(a7, wpy);
-        const float tsv = __fmul_rn(nK1, wpy);
-        float smp[SIDE];
-        unsigned ok = 0;
+        for (int i = 0; i < SIDE; ++i) {
+            const float wpy = fy + static_cast<float>(i * ST - R);
+            const float tqx = __fmul_rn(a1, wpy), tqy = __fmul_rn(a4, wpy), tqz = __fmul_rn(a7, wpy);
+            const float tsv = __fmul_rn(nK1, wpy);
+            float smp[SIDE];
 #pragma unroll
-        for (int j = 0; j < SIDE; ++j) {
-            const float wpx = fx + static_cast<float>(j * ST - R);
-            const float qx = __fadd_rn(__fmaf_rn(a0, wpx, tqx), a2);
-            const float qy = __fadd_rn(__fmaf_rn(a3, wpx, tqy), a5);
-            const float qz = __fadd_rn(__fmaf_rn(a6, wpx, tqz), a8);
-            const float sval = __fadd_rn(__fmaf_rn(nK0, wpx, tsv), nK2);
-            const float factor = __fmul_rn(sval, inv_n_dot_P);
-            const float wz = __fmaf_rn(b2, factor, qz);
-            const float iw = rcp_approx(wz);
-            const float u = __fmul_rn(__fmaf_rn(b0, factor, qx), iw);
-            const float vv = __fmul_rn(__fmaf_rn(b1, factor, qy), iw);
-            const bool skip = fabsf(wz) < 1e-8f || u < 0.0f || u >= fw1 || vv < 0.0f || vv >= fh1;
-            ok |= static_cast<unsigned>(!skip) << j;
-            smp[j] = tex2D<float>(tex, __fadd_rn(u, 0.5f), __fadd_rn(vv, 0.5f));
-        }
-        const float* rrow = s_ref + (ly + i * ST) * tw + lx;
+            for (int j = 0; j < SIDE; ++j) {
+                const float wpx = fx + static_cast<float>(j * ST - R);
+                const float qx = __fadd_rn(__fmaf_rn(a0, wpx, tqx), a2);
+                const float qy = __fadd_rn(__fmaf_rn(a3, wpx, tqy), a5);
+                const float qz = __fadd_rn(__fmaf_rn(a6, wpx, tqz), a8);
+                const float sval = __fadd_rn(__fmaf_rn(nK0, wpx, tsv), nK2);
+                const float factor = __fmul_rn(sval, inv_n_dot_P);
+                const float wz = __fmaf_rn(b2, factor, qz);
+                const float iw = rcp_approx(wz);
+                const float u = __fmul_rn(__fmaf_rn(b0, factor, qx), iw);
+                const float vv = __fmul_rn(__fmaf_rn(b1, factor, qy), iw);
+                smp[j] = tex2D<float>(tex, __fadd_rn(u, 0.5f), __fadd_rn(vv, 0.5f));
+            }
+            const float* rrow = s_ref + (ly + i * ST) * tw + lx;
 #pragma unroll
-        for (int j = 0; j < SIDE; ++j) {
-            if (ok & (1u << j)) {
-                const float rv = rrow[j * ST];
-                const float sv = smp[j];
-                sum_ref = __fadd_rn(sum_ref, rv);
+            for (int j = 0; j < SIDE; ++j) {
+                const float rv = rrow[j * ST], sv = smp[j];
                 sum_src = __fadd_rn(sum_src, sv);
-                sum_ref2 = __fmaf_rn(rv, rv, sum_ref2);
                 sum_src2 = __fmaf_rn(sv, sv, sum_src2);
                 sum_rs = __fmaf_rn(rv, sv, sum_rs);
-                count++;
+            }
+        }
+    } else {
+#pragma unroll 1
+        for (int i = 0; i < SIDE; ++i) {
+            const float wpy = fy + static_cast<float>(i * ST - R);
+            const float tqx = __fmul_rn(a1, wpy), tqy = __fmul_rn(a4, wpy), tqz = __fmul_rn(a7, wpy);
+            const float tsv = __fmul_rn(nK1, wpy);
+            float smp[SIDE];
+            unsigned ok = 0;
+#pragma unroll
+            for (int j = 0; j < SIDE; ++j) {
+                const float wpx = fx + static_cast<float>(j * ST - R);
+                const float qx = __fadd_rn(__fmaf_rn(a0, wpx, tqx), a2);
+                const float qy = __fadd_rn(__fmaf_rn(a3, wpx, tqy), a5);
+                const float qz = __fadd_rn(__fmaf_rn(a6, wpx, tqz), a8);
+                const float sval = __fadd_rn(__fmaf_rn(nK0, wpx, tsv), nK2);
+                const float factor = __fmul_rn(sval, inv_n_dot_P);
+                const float wz = __fmaf_rn(b2, factor, qz);
+                const float iw = rcp_approx(wz);
+                const float u = __fmul_rn(__fmaf_rn(b0, factor, qx), iw);
+                const float vv = __fmul_rn(__fmaf_rn(b1, factor, qy), iw);
+                const bool skip = fabsf(wz) < 1e-8f || u < 0.0f || u >= fw1 || vv < 0.0f || vv >= fh1;
+                ok |= static_cast<unsigned>(!skip) << j;
+                smp[j] = tex2D<float>(tex, __fadd_rn(u, 0.5f), __fadd_rn(vv, 0.5f));
+            }
+            const float* rrow = s_ref + (ly + i * ST) * tw + lx;
+#pragma unroll
+            for (int j = 0; j < SIDE; ++j) {
+                if (ok & (1u << j)) {
+                    const float rv = rrow[j * ST];
+                    const float sv = smp[j];
+                    sum_ref = __fadd_rn(sum_ref, rv);
+                    sum_src = __fadd_rn(sum_src, sv);
+                    sum_ref2 = __fmaf_rn(rv, rv, sum_ref2);
+                    sum_src2 = __fmaf_rn(sv, sv, sum_src2);
+                    sum_rs = __fmaf_rn(rv, sv, sum_rs);
+                    count++;
+                }
             }
         }
     }
@@ -217,6 +291,8 @@ __device__ __forceinline__ float cost_f32(const float* __restrict__ s_ref, int t
     if (count < min_count) {
         c = 2.0f;
     } else {
+        // Opaque: one copy of the expressions below for both branches above, so one choice of fused products.
+        asm volatile("" : "+r"(count));
         const float fc = static_cast<float>(count);
         const float num = fc * sum_rs - sum_ref * sum_src;
         const float den_r = fc * sum_ref2 - sum_ref * sum_ref;
@@ -229,7 +305,7 @@ __device__ __forceinline__ float cost_f32(const float* __restrict__ s_ref, int t
             c = 1.0f - ncc;
         }
     }
-    return c;
+    return sampled ? c : 2.0f;
 }
 
 __global__ void __launch_bounds__(256) init_kernel(BatchList bl) {
@@ -257,13 +333,14 @@ __device__ __forceinline__ void tile_cost(const ViewDesc* v, int tile_x, int til
     // Lanes own consecutive pixels (two 32-pixel halves of the tile row): a
     // warp's taps of one window position then lie next to each other.
     for (int j = 0; j < 2; ++j) {
-        const int lx = 32 * j + lane, x = x0 + lx;
-        if (x >= v->W) continue;
+        // Whole warps score; lanes past the image repeat its last column.
+        const int lx = min(32 * j + lane, v->W - 1 - x0), x = x0 + lx;
+        if (lx < 32 * j) break;
         const size_t idx = static_cast<size_t>(y) * v->W + x;
         const PlaneF32 p = plane_f32(v, x, y, v->hyp[idx]);
+        const float2 sums = window_sums<R, ST>(s_ref, tw, lx, ly);
         Lowest low;
-        if (p.ok)
-            for (int s = 0; s < v->S; ++s) low.insert(cost_f32<R, ST>(s_ref, tw, lx, ly, x, y, p, v, s));
+        for (int s = 0; s < v->S; ++s) low.insert(cost_f32<R, ST>(s_ref, tw, lx, ly, x, y, p, sums, v, s));
         v->cost[idx] = mean_f32(low.sum(min(sc.top_k, v->S)), min(sc.top_k, v->S));
     }
 }
@@ -281,28 +358,31 @@ struct Shared32 {
     float4 plane[CTA_THREADS];  // nK and 1 / (n.P) of the chunk's items
     float unit[HP_MAX_SOURCES * CTA_THREADS];
     unsigned char ok[CTA_THREADS];
+    float2 sums[CTA_THREADS];   // window_sums of each thread's pixel
     PassShared<CTA_THREADS> pass;
 };
 
 // Scorer of the half-pass (red_black_pass).
 template <int R, int ST>
 struct Scorer32 {
+    static constexpr bool WHOLE_WARPS = true;
     const ViewDesc* v;
     const float* s_ref;
     Shared32& sm;
     int x0, y0;
-    __device__ __forceinline__ void begin(int, int) {}
+    __device__ __forceinline__ void begin(int lx, int ly) {
+        sm.sums[threadIdx.x] = window_sums<R, ST>(s_ref, TILE_W + 2 * R, lx, ly);
+    }
     __device__ __forceinline__ void publish() {}
     __device__ __forceinline__ void set_plane(int k, int x, int y, float4 h, bool ok) {
         const PlaneF32 p = plane_f32(v, x, y, h);
         sm.plane[k] = make_float4(p.nK0, p.nK1, p.nK2, p.inv_n_dot_P);
         sm.ok[k] = ok && p.ok;
     }
-    __device__ __forceinline__ float score(int s, int k, int, int lx, int ly) const {
-        if (!sm.ok[k]) return 2.0f;
+    __device__ __forceinline__ float score(int s, int k, int o, int lx, int ly) const {
         const float4 q = sm.plane[k];
-        return cost_f32<R, ST>(s_ref, TILE_W + 2 * R, lx, ly, x0 + lx, y0 + ly, PlaneF32{q.x, q.y, q.z, q.w, true}, v,
-                               s);
+        return cost_f32<R, ST>(s_ref, TILE_W + 2 * R, lx, ly, x0 + lx, y0 + ly, PlaneF32{q.x, q.y, q.z, q.w, sm.ok[k] != 0},
+                               sm.sums[o], v, s);
     }
     __device__ __forceinline__ float mean(float sum, int k) const { return mean_f32(sum, k); }
 };
