@@ -24,11 +24,6 @@
 #include "hp_pass.cuh"
 #include "hp_tile.cuh"
 
-// Resident CTAs per SM the cost kernels are register-budgeted for.
-#ifndef HP_F32_MIN_BLOCKS
-#define HP_F32_MIN_BLOCKS 3
-#endif
-
 namespace hp {
 
 #ifdef HP_COUNT_TAPS
@@ -44,6 +39,15 @@ unsigned long long f32_taps() {
 #endif
 
 namespace {
+
+// Resident CTAs per SM the half-pass is register-budgeted for.  A window row's
+// fetches are in flight together, so up to 8 taps a row 64 registers hold them
+// (2 x 1920 x 1080, r 7, s 2: 97.9 ms, against 99.9 with 3 CTAs and 108.8 with
+// 2); longer rows want 80 (5 x 640 x 480, r 5, s 1: 45.9 ms with 3 or 4, 48.3
+// with 2; one 320 x 240 view 1247, 1276 and 1262 us with 3, 4 and 2).
+template <int R, int ST>
+constexpr int pass_blocks() { return (2 * R) / ST + 1 <= 8 ? 4 : 3; }
+constexpr int COST_BLOCKS = 3;  // full-map cost, 1920 x 1080, r 5, s 1: 1486 us, 1574 with 2, 1506 with 4
 
 constexpr int MAX_TW = TILE_W + 2 * HP_MAX_RADIUS;
 constexpr int MAX_TH = TILE_H + 2 * HP_MAX_RADIUS;
@@ -346,7 +350,7 @@ __device__ __forceinline__ void tile_cost(const ViewDesc* v, int tile_x, int til
 }
 
 template <int R, int ST>
-__global__ void __launch_bounds__(CTA_THREADS, HP_F32_MIN_BLOCKS) cost_kernel(BatchList bl, SolveConsts sc) {
+__global__ void __launch_bounds__(CTA_THREADS, COST_BLOCKS) cost_kernel(BatchList bl, SolveConsts sc) {
     __shared__ float s_ref[MAX_TW * MAX_TH];
     int tile_x, tile_y;
     const ViewDesc* v = locate_tile(bl, blockIdx.x, &tile_x, &tile_y);
@@ -398,8 +402,9 @@ __device__ __forceinline__ void tile_propagate(const ViewDesc* v, int tile_x, in
 }
 
 template <int R, int ST>
-__global__ void __launch_bounds__(CTA_THREADS, HP_F32_MIN_BLOCKS) propagate_kernel(BatchList bl, SolveConsts sc,
-                                                                                   int iteration, int color) {
+__global__ void __launch_bounds__(CTA_THREADS, pass_blocks<R, ST>()) propagate_kernel(BatchList bl,
+                                                                                         SolveConsts sc, int iteration,
+                                                                                         int color) {
     __shared__ float s_ref[MAX_TW * MAX_TH];
     __shared__ Shared32 sm;
     int tile_x, tile_y;
@@ -412,7 +417,7 @@ __global__ void __launch_bounds__(CTA_THREADS, HP_F32_MIN_BLOCKS) propagate_kern
 // bodies are the functions the per-stage kernels above run, so the results
 // are bit-identical to the per-stage launch sequence.
 template <int R, int ST>
-__global__ void __launch_bounds__(CTA_THREADS, HP_F32_MIN_BLOCKS) persistent_kernel(Schedule s) {
+__global__ void __launch_bounds__(CTA_THREADS, pass_blocks<R, ST>()) persistent_kernel(Schedule s) {
     __shared__ float s_ref[MAX_TW * MAX_TH];
     __shared__ Shared32 sm;
     // The claimed tile lives in shared memory: thread 0 decodes it once and

@@ -67,9 +67,22 @@ struct PassShared {
     int survivors;
 };
 
-// One half-pass of the tile at (x0, y0): TILE_W x NT / 32 pixels, thread
-// (row, lane) owns pixel x0 + 2 * lane + ((y + color) & 1) of row y0 + row, so
-// every thread has work, where the reference idles half its grid.
+// Tile position of thread t's pixel (the active pixels of a TILE_W x NT / 32
+// tile).  A warp covers a 32 x 2 block, four lanes a 4 x 2 block of it: the
+// texture unit takes a fetch by fours, and their footprints then share a few
+// texels, where four pixels two apart in one row spread over a 7 x 1 run (FP32,
+// 2 x 1920 x 1080, r 7, s 2: 106.9 -> 100.0 ms; 16 x 4 and 8 x 8 warps measure
+// the same there).  The software sampler prefers wide blocks, whose rows of
+// quads fill L1 lines: FP16-acc, 4 views, 32 x 2 128.4 ms, one row 128.1, 16 x 4
+// 132.1, 8 x 8 133.8; with r 5, s 1 32 x 2 is the best, 55.1 ms against 56.3.
+__device__ __forceinline__ int2 pass_pixel(int t, int y0, int color) {
+    const int ly = ((t >> 6) << 1) | ((t >> 1) & 1);
+    const int lx = (t & 32) + 4 * ((t & 31) >> 2) + 2 * (t & 1) + ((y0 + ly + color) & 1);
+    return make_int2(lx, ly);
+}
+
+// One half-pass of the tile at (x0, y0), TILE_W x NT / 32 pixels: every thread
+// owns an active pixel, where the reference idles half its grid.
 // The scorer K, per thread:
 //   begin(lx, ly)               prepares the window of the thread's own pixel (active pixels only)
 //   publish()                   makes it readable by the other threads (after the next barrier)
@@ -82,10 +95,11 @@ __device__ __forceinline__ void red_black_pass(const ViewDesc* v, int x0, int y0
                                                int iteration, int color, K& scorer, float* unit,
                                                PassShared<NT>& sm) {
     const int W = v->W, H = v->H, S = v->S;
-    const int tid = threadIdx.x, ly = tid >> 5, lane = tid & 31;
-    const int y = y0 + ly;
-    const int lx = 2 * lane + ((y + color) & 1);
-    const int x = x0 + lx;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int2 own = pass_pixel(tid, y0, color);
+    const int lx = own.x, ly = own.y, x = x0 + lx, y = y0 + ly;
+    // Read through a broadcast: the compiler then knows that it is the same for a warp's lanes.
+    const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const bool active = y < H && x < W;  // every thread takes part in the barriers
     const size_t idx = static_cast<size_t>(y) * W + x;
     float4 best = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -107,7 +121,7 @@ __device__ __forceinline__ void red_black_pass(const ViewDesc* v, int x0, int y0
         const int t = __shfl_up_sync(0xffffffffu, incl, o);
         if (lane >= o) incl += t;
     }
-    if (lane == 31) sm.warp_total[ly] = incl;
+    if (lane == 31) sm.warp_total[warp] = incl;
     __syncthreads();
     int total = 0;
     {
@@ -115,7 +129,7 @@ __device__ __forceinline__ void red_black_pass(const ViewDesc* v, int x0, int y0
 #pragma unroll
         for (int w = 0; w < NT / 32; ++w) {
             const int t = sm.warp_total[w];
-            k += w < ly ? t : 0;
+            k += w < warp ? t : 0;
             total += t;
         }
         for (int cand = 0; cand < 4; ++cand)
@@ -125,7 +139,6 @@ __device__ __forceinline__ void red_black_pass(const ViewDesc* v, int x0, int y0
     // Values that steer the loops below, read through a broadcast: the compiler then knows that a warp stays together
     // in them, and a texture handle stays in a uniform register (with a scorer's votes inside it is otherwise fetched
     // lane by lane: FP32, 2 x 1920 x 1080, 149.7 ms against 115.1).
-    const int warp = __shfl_sync(0xffffffffu, ly, 0);
     total = __shfl_sync(0xffffffffu, total, 0);
     const int kk = min(sc.top_k, S), lead = S - kk + 1;
     float drange = __fmul_rn(__fsub_rn(v->dmax, v->dmin), 0.5f);
@@ -167,7 +180,8 @@ __device__ __forceinline__ void red_black_pass(const ViewDesc* v, int x0, int y0
             } else if (tid < n) {
                 item = sm.items[c0 + tid];
                 const int o = item >> 2, cand = item & 3;
-                const int oy = y0 + (o >> 5), ox = x0 + 2 * (o & 31) + ((oy + color) & 1);
+                const int2 at = pass_pixel(o, y0, color);
+                const int ox = x0 + at.x, oy = y0 + at.y;
                 const int nxp = ox + (cand == 0 ? -1 : (cand == 1 ? 1 : 0));
                 const int nyp = oy + (cand == 2 ? -1 : (cand == 3 ? 1 : 0));
                 float4 h = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -194,8 +208,8 @@ __device__ __forceinline__ void red_black_pass(const ViewDesc* v, int x0, int y0
                         if (!K::WHOLE_WARPS && u >= units) continue;
                         const int k = first > 0 ? sm.items[u] : u;
                         const int o = round == 0 ? sm.items[c0 + k] >> 2 : k;
-                        const int oly = o >> 5;
-                        unit[q * NT + k] = scorer.score(source, k, o, 2 * (o & 31) + ((y0 + oly + color) & 1), oly);
+                        const int2 at = pass_pixel(o, y0, color);
+                        unit[q * NT + k] = scorer.score(source, k, o, at.x, at.y);
                     }
                 }
                 __syncthreads();  // the part's source costs are complete
