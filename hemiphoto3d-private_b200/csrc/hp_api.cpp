@@ -943,11 +943,11 @@ hp_status hp_fuse_depth_maps(hp_ctx* ctx, const hp_fuse_view* views, int num_vie
         hp::FuseView& f = fv[i];
         std::memset(&f, 0, sizeof f);
         for (int k = 0; k < 9; ++k) {
-            f.K[k] = static_cast<float>(v.cam.K[k]);
-            f.kinv[k] = static_cast<float>(kinv[k]);
-            f.R[k] = static_cast<float>(v.cam.R[k]);
+            f.cam.K[k] = static_cast<float>(v.cam.K[k]);
+            f.cam.kinv[k] = static_cast<float>(kinv[k]);
+            f.cam.R[k] = static_cast<float>(v.cam.R[k]);
         }
-        for (int k = 0; k < 3; ++k) f.t[k] = static_cast<float>(v.cam.t[k]);
+        for (int k = 0; k < 3; ++k) f.cam.t[k] = static_cast<float>(v.cam.t[k]);
         f.W = v.width;
         f.H = v.height;
         f.nb_begin = static_cast<int>(nbs.size());
@@ -966,10 +966,9 @@ hp_status hp_fuse_depth_maps(hp_ctx* ctx, const hp_fuse_view* views, int num_vie
         f.nb_count = static_cast<int>(nbs.size()) - f.nb_begin;
         vblock[i] = static_cast<int>(blocks);
         const size_t px = static_cast<size_t>(v.width) * v.height;
-        blocks += static_cast<long long>((px + hp::FUSE_THREADS - 1) / hp::FUSE_THREADS);
-        // The one-CTA scan splits the per-CTA counts into 1024 chunks with int
-        // offsets; 2^30 CTAs (2.7e11 pixels) keeps those offsets in range.
-        if (blocks > (1ll << 30)) return fail(ctx, HP_ERR_INVALID_ARG, "fuse: too many pixels");
+        blocks += static_cast<long long>((px + hp::FUSE_PIXELS - 1) / hp::FUSE_PIXELS);
+        // The one-CTA scan indexes the per-CTA counts with ints; 2^28 CTAs (2.7e11 pixels) keep them in range.
+        if (blocks > (1ll << 28)) return fail(ctx, HP_ERR_INVALID_ARG, "fuse: too many pixels");
         staged_floats += px * (4 + (v.confidence ? 1 : 0) + (v.gray ? 1 : 0));
     }
     vblock[num_views] = static_cast<int>(blocks);
@@ -999,11 +998,12 @@ hp_status hp_fuse_depth_maps(hp_ctx* ctx, const hp_fuse_view* views, int num_vie
             HP_CUDA(stage(views[i].gray, px, &fv[i].gray));
         }
     }
-    // Descriptor block: views | neighbours | first CTA per view | CTA counts | CTA offsets | total.
+    // Descriptor block: views | neighbours | first CTA per view | ballots | CTA counts | CTA offsets | total.
     auto up8 = [](size_t b) { return (b + 7) / 8 * 8; };
     const size_t o_nb = up8(sizeof(hp::FuseView) * num_views);
     const size_t o_vb = o_nb + up8(sizeof(int) * std::max<size_t>(nbs.size(), 1));
-    const size_t o_cnt = o_vb + up8(sizeof(int) * (num_views + 1));
+    const size_t o_bal = o_vb + up8(sizeof(int) * (num_views + 1));
+    const size_t o_cnt = o_bal + sizeof(unsigned) * (hp::FUSE_PIXELS / 32) * blocks;
     const size_t o_off = o_cnt + up8(sizeof(int) * blocks);
     const size_t o_tot = o_off + sizeof(long long) * blocks;
     Scratch desc;
@@ -1025,11 +1025,12 @@ hp_status hp_fuse_depth_maps(hp_ctx* ctx, const hp_fuse_view* views, int num_vie
     a.max_depth_rel = prm->max_depth_rel;
     a.max_reproj_sq = prm->max_reproj_px * prm->max_reproj_px;
     a.min_normal_cos = prm->min_normal_cos;
+    unsigned* ballots = reinterpret_cast<unsigned*>(base + o_bal);
     int* counts = reinterpret_cast<int*>(base + o_cnt);
     long long* offsets = reinterpret_cast<long long*>(base + o_off);
     long long* d_total = reinterpret_cast<long long*>(base + o_tot);
     const int nb = static_cast<int>(blocks);
-    HP_CUDA(counted(ctx, HP_KERNEL_OTHER, [&] { return hp::launch_fuse_count(a, nb, counts, ctx->stream); }));
+    HP_CUDA(counted(ctx, HP_KERNEL_OTHER, [&] { return hp::launch_fuse_count(a, nb, ballots, counts, ctx->stream); }));
     HP_CUDA(counted(ctx, HP_KERNEL_OTHER,
                     [&] { return hp::launch_fuse_scan(counts, nb, offsets, d_total, ctx->stream); }));
     long long total = 0;
@@ -1040,7 +1041,7 @@ hp_status hp_fuse_depth_maps(hp_ctx* ctx, const hp_fuse_view* views, int num_vie
     if (nw > 0 && (out->positions || out->normals || out->colors)) {
         if (out->memory == HP_MEMORY_DEVICE) {
             HP_CUDA(counted(ctx, HP_KERNEL_OTHER, [&] {
-                return hp::launch_fuse_write(a, nb, offsets, out->positions, out->normals, out->colors, nw,
+                return hp::launch_fuse_write(a, nb, ballots, offsets, out->positions, out->normals, out->colors, nw,
                                              ctx->stream);
             }));
         } else {  // written on the device, then copied out
@@ -1051,7 +1052,7 @@ hp_status hp_fuse_depth_maps(hp_ctx* ctx, const hp_fuse_view* views, int num_vie
             float* tn = tp + per;
             float* tc = tn + per;
             HP_CUDA(counted(ctx, HP_KERNEL_OTHER, [&] {
-                return hp::launch_fuse_write(a, nb, offsets, out->positions ? tp : nullptr,
+                return hp::launch_fuse_write(a, nb, ballots, offsets, out->positions ? tp : nullptr,
                                              out->normals ? tn : nullptr, out->colors ? tc : nullptr, nw,
                                              ctx->stream);
             }));

@@ -181,13 +181,17 @@ struct FilterMaps {
 };
 
 // Depth-map fusion (hp_fuse_depth_maps): one view's device maps and its
-// camera cast to FP32 (kinv is the FP64 inverse of K, then cast).
-struct FuseView {
+// camera cast to FP32 (kinv is the FP64 inverse of K, then cast).  The camera
+// is read as eight 16-byte words.
+struct FuseCamera {
+    float K[9], kinv[9], R[9], t[3], pad[2];
+};
+struct alignas(16) FuseView {
+    FuseCamera cam;
     const float* depth;
     const float* normal;
     const float* conf;  // may be null
     const float* gray;  // may be null
-    float K[9], kinv[9], R[9], t[3];
     int W, H;
     int nb_begin, nb_count;  // this view's slice of FuseArgs::neighbors
 };
@@ -199,7 +203,8 @@ struct FuseArgs {
     int min_views;
     float min_conf, max_depth_rel, max_reproj_sq, min_normal_cos;
 };
-constexpr int FUSE_THREADS = 256;  // pixels per CTA of the fusion kernels
+constexpr int FUSE_THREADS = 256;
+constexpr int FUSE_PIXELS = 1024;  // pixels per CTA of the fusion kernels, in four steps of FUSE_THREADS
 
 }  // namespace hp
 
@@ -239,11 +244,13 @@ cudaError_t launch_filter_maps(const FilterMaps& a, float* depth, const float* n
                                cudaStream_t st);
 cudaError_t launch_to_f32(const void* src, int dtype, int W, int H, float* dst, int dst_pitch, __half* dst16,
                           int dst16_pitch, cudaStream_t st);
-// Fusion: per-CTA counts of emitted points, their exclusive prefix (and the
-// total), then the points written at their offsets (index < capacity only).
-cudaError_t launch_fuse_count(const FuseArgs& a, int blocks, int* block_counts, cudaStream_t st);
+// Fusion: per CTA the emitted pixels (FUSE_PIXELS / 32 ballot words) and their
+// number, the numbers' exclusive prefix (and the total), then the points
+// written at their offsets (index < capacity only).
+cudaError_t launch_fuse_count(const FuseArgs& a, int blocks, unsigned* ballots, int* block_counts, cudaStream_t st);
 cudaError_t launch_fuse_scan(const int* block_counts, int blocks, long long* block_offsets, long long* total,
                              cudaStream_t st);
-cudaError_t launch_fuse_write(const FuseArgs& a, int blocks, const long long* block_offsets, float* positions,
-                              float* normals, float* colors, long long capacity, cudaStream_t st);
+cudaError_t launch_fuse_write(const FuseArgs& a, int blocks, const unsigned* ballots,
+                              const long long* block_offsets, float* positions, float* normals, float* colors,
+                              long long capacity, cudaStream_t st);
 }  // namespace hp

@@ -109,7 +109,7 @@ __device__ __forceinline__ void red_black_pass(const ViewDesc* v, int x0, int y0
     if (active) {
         scorer.begin(lx, ly);
         best = v->hyp[idx];
-        best_cost = cost_value(v->cost[idx]);
+        best_cost = sc.memo ? cost_value(v->cost[idx]) : v->cost[idx];  // a caller's cost as it is
         need = neighbour_needs(v, x, y, best, sc.memo && iteration > 0);
     }
     scorer.publish();
