@@ -627,7 +627,7 @@ __global__ void __launch_bounds__(Tile<TH>::NT, Tile<TH>::MIN_BLOCKS) cost16_ker
 template <int R, int ST, int TH, int D>
 struct Scorer16 {
     static constexpr int NT = Tile<TH>::NT, TW = TILE_W + 2 * R;
-    static constexpr bool WHOLE_WARPS = false;
+    static constexpr bool BLOCKS = !Win<R, ST>::IN_SMEM, BY_PLANE = false, WHOLE_WARPS = false;
     const ViewDesc* v;
     Shared<R, ST, TH>& sm;
     int x0, y0;

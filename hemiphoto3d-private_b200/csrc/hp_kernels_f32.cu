@@ -369,7 +369,7 @@ struct Shared32 {
 // Scorer of the half-pass (red_black_pass).
 template <int R, int ST>
 struct Scorer32 {
-    static constexpr bool WHOLE_WARPS = true;
+    static constexpr bool BLOCKS = true, BY_PLANE = true, WHOLE_WARPS = true;
     const ViewDesc* v;
     const float* s_ref;
     Shared32& sm;

@@ -63,22 +63,36 @@ template <int NT>
 struct PassShared {
     float cost[NT * 4];            // neighbour costs, slot (thread << 2 | cand)
     unsigned short items[NT * 4];  // neighbour items (thread << 2 | cand), then the surviving trials
+    unsigned char need[NT];        // neighbour planes each thread's pixel scores (bit per cand)
     int warp_total[NT / 32];
     int survivors;
 };
 
 // Tile position of thread t's pixel (the active pixels of a TILE_W x NT / 32
-// tile).  A warp covers a 32 x 2 block, four lanes a 4 x 2 block of it: the
+// tile), by rows or by blocks.
+// Blocks: a warp covers 32 x 2 pixels, four lanes a 4 x 2 block of them.  The
 // texture unit takes a fetch by fours, and their footprints then share a few
 // texels, where four pixels two apart in one row spread over a 7 x 1 run (FP32,
 // 2 x 1920 x 1080, r 7, s 2: 106.9 -> 100.0 ms; 16 x 4 and 8 x 8 warps measure
-// the same there).  The software sampler prefers wide blocks, whose rows of
-// quads fill L1 lines: FP16-acc, 4 views, 32 x 2 128.4 ms, one row 128.1, 16 x 4
-// 132.1, 8 x 8 133.8; with r 5, s 1 32 x 2 is the best, 55.1 ms against 56.3.
+// the same there).
+// Rows: a warp covers 64 pixels of one row.  The software sampler's quads lie in
+// rows, and a warp in one row touches the fewest L1 lines (FP16-acc, r 7, s 2,
+// rows / 32 x 2 / 16 x 4 / 8 x 8: 4 x 1920 x 1080 128.0 / 129.2 / 132.1 / 133.8
+// ms; 5 and 6 uneven views in persistent launches 32.6 and 80.3 ms against 33.7
+// and 83.7).  Its windows beyond shared memory (r 5, s 1) also read the reference
+// tile, and take blocks: 56.3 / 55.1 / 56.7 / 58.7 ms.
+template <bool BLOCKS>
 __device__ __forceinline__ int2 pass_pixel(int t, int y0, int color) {
-    const int ly = ((t >> 6) << 1) | ((t >> 1) & 1);
-    const int lx = (t & 32) + 4 * ((t & 31) >> 2) + 2 * (t & 1) + ((y0 + ly + color) & 1);
-    return make_int2(lx, ly);
+    const int ly = BLOCKS ? ((t >> 6) << 1) | ((t >> 1) & 1) : t >> 5;
+    const int lx = BLOCKS ? (t & 32) + 4 * ((t & 31) >> 2) + 2 * (t & 1) : 2 * (t & 31);
+    return make_int2(lx + ((y0 + ly + color) & 1), ly);
+}
+
+// The thread that owns the active pixel at tile position (lx, ly).
+template <bool BLOCKS>
+__device__ __forceinline__ int pass_thread(int lx, int ly) {
+    return BLOCKS ? ((ly >> 1) << 6) | (lx & 32) | (((lx & 31) >> 2) << 2) | ((ly & 1) << 1) | ((lx >> 1) & 1)
+                  : ly << 5 | lx >> 1;
 }
 
 // One half-pass of the tile at (x0, y0), TILE_W x NT / 32 pixels: every thread
@@ -89,6 +103,8 @@ __device__ __forceinline__ int2 pass_pixel(int t, int y0, int color) {
 //   set_plane(k, x, y, h, ok)   thread k: plane h of item k at pixel (x, y), ok false: no plane
 //   score(source, k, o, lx, ly) cost of item k, whose pixel is thread o's, at tile position (lx, ly)
 //   mean(sum, k)                sum / k, monotone in sum
+//   BLOCKS                      pass_pixel's layout
+//   BY_PLANE                    neighbour items are listed by the plane they score, not by pixel
 //   WHOLE_WARPS                 score needs all 32 lanes of a warp together
 template <int NT, class K>
 __device__ __forceinline__ void red_black_pass(const ViewDesc* v, int x0, int y0, const SolveConsts& sc,
@@ -96,7 +112,7 @@ __device__ __forceinline__ void red_black_pass(const ViewDesc* v, int x0, int y0
                                                PassShared<NT>& sm) {
     const int W = v->W, H = v->H, S = v->S;
     const int tid = threadIdx.x, lane = tid & 31;
-    const int2 own = pass_pixel(tid, y0, color);
+    const int2 own = pass_pixel<K::BLOCKS>(tid, y0, color);
     const int lx = own.x, ly = own.y, x = x0 + lx, y = y0 + ly;
     // Read through a broadcast: the compiler then knows that it is the same for a warp's lanes.
     const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
@@ -113,8 +129,32 @@ __device__ __forceinline__ void red_black_pass(const ViewDesc* v, int x0, int y0
         need = neighbour_needs(v, x, y, best, sc.memo && iteration > 0);
     }
     scorer.publish();
+    // Neighbour items are listed by pixel (bit 4 + c of `list`: the own pixel's neighbour c), or by plane: thread t
+    // lists the tile's pixels around the inactive pixel of its own 2-pixel cell (bit c: the pixel whose neighbour c that
+    // one is), then its own pixel's planes from outside the tile.  The up to four items of a plane are then adjacent
+    // lanes, whose windows nearly coincide in every source.  That suits the texture unit (2 x 1920 x 1080, r 7, s 2:
+    // 97.9 -> 90.7 ms, 5 x 640 x 480, r 5, s 1: 45.7 -> 42.1 ms), while the software sampler is better off with the
+    // planes of one pixel, whose windows keep to its rows of quads (4 x 1920 x 1080: 129.2 ms, by plane 136.6).
+    unsigned list = need << 4;
+    const int nx = lx ^ 1, ny = ly;  // tiles start at even columns: the cell is columns lx, lx ^ 1
+    auto owner = [&](int c) {
+        return pass_thread<K::BLOCKS>(nx + (c == 0 ? 1 : (c == 1 ? -1 : 0)), ny + (c == 2 ? 1 : (c == 3 ? -1 : 0)));
+    };
+    if constexpr (K::BY_PLANE) {
+        sm.need[tid] = static_cast<unsigned char>(need);
+        __syncthreads();
+        list = 0;
+        constexpr int TH = NT / 32;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const bool in = c == 0 ? nx + 1 < TILE_W : (c == 1 ? nx > 0 : (c == 2 ? ny + 1 < TH : ny > 0));
+            if (in && ((sm.need[owner(c)] >> c) & 1u)) list |= 1u << c;
+            const bool outside = c == 0 ? lx == 0 : (c == 1 ? lx + 1 == TILE_W : (c == 2 ? ly == 0 : ly + 1 == TH));
+            if (outside && ((need >> c) & 1u)) list |= 16u << c;
+        }
+    }
     // Exclusive scan of the item counts over the warp, then over the CTA's warps.
-    const int cnt = __popc(need);
+    const int cnt = __popc(list);
     int incl = cnt;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -132,8 +172,10 @@ __device__ __forceinline__ void red_black_pass(const ViewDesc* v, int x0, int y0
             k += w < warp ? t : 0;
             total += t;
         }
-        for (int cand = 0; cand < 4; ++cand)
-            if (need & (1u << cand)) sm.items[k++] = static_cast<unsigned short>((tid << 2) | cand);
+        for (int c = 0; K::BY_PLANE && c < 4; ++c)
+            if (list & (1u << c)) sm.items[k++] = static_cast<unsigned short>((owner(c) << 2) | c);
+        for (int c = 0; c < 4; ++c)
+            if (list & (16u << c)) sm.items[k++] = static_cast<unsigned short>((tid << 2) | c);
     }
     __syncthreads();  // the item list is complete
     // Values that steer the loops below, read through a broadcast: the compiler then knows that a warp stays together
@@ -180,7 +222,7 @@ __device__ __forceinline__ void red_black_pass(const ViewDesc* v, int x0, int y0
             } else if (tid < n) {
                 item = sm.items[c0 + tid];
                 const int o = item >> 2, cand = item & 3;
-                const int2 at = pass_pixel(o, y0, color);
+                const int2 at = pass_pixel<K::BLOCKS>(o, y0, color);
                 const int ox = x0 + at.x, oy = y0 + at.y;
                 const int nxp = ox + (cand == 0 ? -1 : (cand == 1 ? 1 : 0));
                 const int nyp = oy + (cand == 2 ? -1 : (cand == 3 ? 1 : 0));
@@ -208,7 +250,7 @@ __device__ __forceinline__ void red_black_pass(const ViewDesc* v, int x0, int y0
                         if (!K::WHOLE_WARPS && u >= units) continue;
                         const int k = first > 0 ? sm.items[u] : u;
                         const int o = round == 0 ? sm.items[c0 + k] >> 2 : k;
-                        const int2 at = pass_pixel(o, y0, color);
+                        const int2 at = pass_pixel<K::BLOCKS>(o, y0, color);
                         unit[q * NT + k] = scorer.score(source, k, o, at.x, at.y);
                     }
                 }
