@@ -672,12 +672,15 @@ __global__ void __launch_bounds__(Tile<TH>::NT, Tile<TH>::MIN_BLOCKS) propagate1
 template <int R, int ST, int TH, int D>
 __global__ void __launch_bounds__(Tile<TH>::NT, Tile<TH>::MIN_BLOCKS) persistent16_kernel(Schedule s) {
     Shared<R, ST, TH>& sm = shared_of<R, ST, TH>();
-    // The claimed tile lives in shared memory: thread 0 decodes it once and
-    // publishes it after the stage, so no thread carries it through the body.
+    // The claimed tile lives in shared memory: warp 0 decodes it once and
+    // thread 0 publishes it after the stage, so no thread carries it through the body.
     __shared__ SchedTile s_tile;
     __shared__ int s_ok;
     for (;;) {
-        if (threadIdx.x == 0) s_ok = sched_claim(s, &s_tile);
+        if (threadIdx.x < 32) {
+            const bool ok = sched_claim(s, &s_tile);
+            if (threadIdx.x == 0) s_ok = ok;
+        }
         __syncthreads();
         if (!s_ok) break;
         // Rebuilt from the kernel parameter rather than read back from shared

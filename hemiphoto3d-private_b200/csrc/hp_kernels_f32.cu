@@ -420,12 +420,15 @@ template <int R, int ST>
 __global__ void __launch_bounds__(CTA_THREADS, pass_blocks<R, ST>()) persistent_kernel(Schedule s) {
     __shared__ float s_ref[MAX_TW * MAX_TH];
     __shared__ Shared32 sm;
-    // The claimed tile lives in shared memory: thread 0 decodes it once and
-    // publishes it after the stage, so no thread carries it through the body.
+    // The claimed tile lives in shared memory: warp 0 decodes it once and
+    // thread 0 publishes it after the stage, so no thread carries it through the body.
     __shared__ SchedTile s_tile;
     __shared__ int s_ok;
     for (;;) {
-        if (threadIdx.x == 0) s_ok = sched_claim(s, &s_tile);
+        if (threadIdx.x < 32) {
+            const bool ok = sched_claim(s, &s_tile);
+            if (threadIdx.x == 0) s_ok = ok;
+        }
         __syncthreads();
         if (!s_ok) break;
         // Rebuilt from the kernel parameter rather than read back from shared

@@ -168,11 +168,20 @@ __device__ __forceinline__ unsigned ld_acquire_gpu_u32(const unsigned* p) {
     return v;
 }
 
+// Claiming is the work of warp 0, all its lanes together: between a CTA's stages
+// its other warps wait for it, so its chain of memory accesses is kept short.
+// The ticket's entry is found 32 probes at a time and the dependencies' flags
+// are polled by a lane each, where one thread took a binary search and up to
+// five polls in a row (FIGURES).
 __device__ __forceinline__ SchedTile decode_ticket(const Schedule& s, int t) {
-    int lo = 0, hi = s.n_entries - 1;
-    while (lo < hi) {  // last entry starting at or before t
-        const int mid = (lo + hi + 1) >> 1;
-        if (s.entry_ticket[mid] <= t) lo = mid; else hi = mid - 1;
+    const int lane = threadIdx.x & 31;
+    int lo = 0, n = s.n_entries;
+    while (n > 1) {  // the entry is among [lo, lo + n): the last starting at or before t
+        const int step = (n + 31) >> 5;
+        const bool le = lane * step < n && s.entry_ticket[lo + lane * step] <= t;
+        const int seg = 31 - __clz(__ballot_sync(0xffffffffu, le));
+        lo += seg * step;
+        n = min(step, n - seg * step);
     }
     const int2 info = s.entry_info[lo];
     SchedTile r;
@@ -201,8 +210,8 @@ __device__ __forceinline__ bool sched_aborted(const Schedule& s) {
     return true;
 }
 
-// Bounded poll of thread 0 for `ticket`: spins while ready() is false.
-// Bounded by the schedule's time limit and by a poll count (in case the
+// Bounded poll of warp 0 for `ticket`: spins while ready() is false on any
+// lane.  Bounded by the schedule's time limit and by a poll count (in case the
 // global timer stands still); false when this or another CTA gave up.  The
 // time limit counts only after kMinPolls sleeping polls, so a step of the
 // global timer during a short wait cannot end it.
@@ -214,53 +223,54 @@ struct WaitBudget {
 template <class Ready>
 __device__ __forceinline__ bool sched_poll(const Schedule& s, int ticket, WaitBudget& b, Ready ready) {
     constexpr unsigned kMinPolls = 4096, kMaxPolls = 1u << 26;
-    while (!ready()) {
-        if (sched_aborted(s)) return false;
-        if (++b.polls > 16) {
-            const unsigned long long now = global_ns();
-            if (b.start == 0) b.start = now;
-            if ((now - b.start > s.wait_limit_ns && b.polls > kMinPolls) || b.polls > kMaxPolls) {
-                sched_abort(s, ticket);
-                return false;
+    while (!__all_sync(0xffffffffu, ready())) {
+        bool stop = false;
+        if ((threadIdx.x & 31) == 0) {
+            if (sched_aborted(s)) {
+                stop = true;
+            } else if (++b.polls > 16) {
+                const unsigned long long now = global_ns();
+                if (b.start == 0) b.start = now;
+                if ((now - b.start > s.wait_limit_ns && b.polls > kMinPolls) || b.polls > kMaxPolls) {
+                    sched_abort(s, ticket);
+                    stop = true;
+                } else {
+                    __nanosleep(256);
+                }
             }
-            __nanosleep(256);
         }
+        if (__shfl_sync(0xffffffffu, stop, 0)) return false;
     }
     return true;
 }
 
-// Thread 0 of a CTA: wait until the tile and its 4-neighbour tiles have
-// finished stage - 1.  A filter stage also waits until every ticket of the
-// solve proper has finished and the previous filtered view's stage has
-// finished on all its tiles (both counts only grow, and every ticket they
-// count precedes this one, so each is held by a running CTA).
+// Warp 0 of a CTA: wait until the tile and its 4-neighbour tiles have finished
+// stage - 1 (lanes 0 to 4 poll one each).  A filter stage also waits until
+// every ticket of the solve proper has finished and the previous filtered
+// view's stage has finished on all its tiles (both counts only grow, and every
+// ticket they count precedes this one, so each is held by a running CTA).
 __device__ __forceinline__ bool sched_wait(const Schedule& s, const SchedTile& t) {
     if (t.stage == 0) return true;
     const int need = t.stage - 1;
-    const int* done = t.v->done;
-    const int tx = t.v->tiles_x;
-    int deps[5];
-    int n = 0;
-    deps[n++] = t.tile;
-    if (t.tx > 0) deps[n++] = t.tile - 1;
-    if (t.tx + 1 < tx) deps[n++] = t.tile + 1;
-    if (t.ty > 0) deps[n++] = t.tile - tx;
-    if (t.ty + 1 < t.v->tiles_y) deps[n++] = t.tile + tx;
+    const int lane = threadIdx.x & 31, tx = t.v->tiles_x;
+    const int* flag = nullptr;
+    if (lane == 0) flag = t.v->done + t.tile;
+    if (lane == 1 && t.tx > 0) flag = t.v->done + t.tile - 1;
+    if (lane == 2 && t.tx + 1 < tx) flag = t.v->done + t.tile + 1;
+    if (lane == 3 && t.ty > 0) flag = t.v->done + t.tile - tx;
+    if (lane == 4 && t.ty + 1 < t.v->tiles_y) flag = t.v->done + t.tile + tx;
     WaitBudget b;
-    for (int i = 0; i < n; ++i) {
-        const int* flag = done + deps[i];
-        if (!sched_poll(s, t.ticket, b, [&] { return ld_acquire_gpu(flag) >= need; })) return false;
-    }
+    if (!sched_poll(s, t.ticket, b, [&] { return !flag || ld_acquire_gpu(flag) >= need; })) return false;
     if (s.main_done && is_filter_stage(t.v, t.stage)) {
         const unsigned main_total = static_cast<unsigned>(s.main_total);
-        if (!sched_poll(s, t.ticket, b, [&] { return ld_acquire_gpu_u32(s.main_done) >= main_total; }))
+        if (!sched_poll(s, t.ticket, b, [&] { return lane > 0 || ld_acquire_gpu_u32(s.main_done) >= main_total; }))
             return false;
         const int prev = t.v->filter->prev;
         if (prev >= 0) {
             const ViewDesc* pv = &s.views[prev];
             const int* cnt = pv->filter->tiles_done;
             const int want = pv->tiles_x * pv->tiles_y;
-            if (!sched_poll(s, t.ticket, b, [&] { return ld_acquire_gpu(cnt) >= want; })) return false;
+            if (!sched_poll(s, t.ticket, b, [&] { return lane > 0 || ld_acquire_gpu(cnt) >= want; })) return false;
         }
     }
     return true;
@@ -269,9 +279,10 @@ __device__ __forceinline__ bool sched_wait(const Schedule& s, const SchedTile& t
 // Thread 0, after the CTA's barrier at the end of a stage: publish it.
 __device__ __forceinline__ void sched_publish(const Schedule& s, const SchedTile& t) {
     if (t.view == s.stall_view && t.tile == s.stall_tile) return;
-    __threadfence();
+    // The barrier before this orders the CTA's stores ahead of the release (cumulative at gpu scope).
     st_release_gpu(t.v->done + t.tile, t.stage);
     if (s.main_done) {
+        __threadfence();  // the counts below are relaxed atomics
         if (t.ticket < s.main_total)
             atomicAdd(s.main_done, 1u);
         else if (is_filter_stage(t.v, t.stage))
@@ -279,16 +290,17 @@ __device__ __forceinline__ void sched_publish(const Schedule& s, const SchedTile
     }
 }
 
-// Thread 0: claims the CTA's next ticket and decodes it into *out; false when
-// the schedule is exhausted or aborted (including a dependency wait of this
-// ticket that ran out).
+// Warp 0: claims the CTA's next ticket and decodes it into *out (written by
+// lane 0); false when the schedule is exhausted or aborted (including a
+// dependency wait of this ticket that ran out).
 __device__ __forceinline__ bool sched_claim(const Schedule& s, SchedTile* out) {
-    if (sched_aborted(s)) return false;
-    const int t = static_cast<int>(atomicAdd(s.counter, 1u));
-    if (t >= s.total) return false;
+    int t = -1;
+    if ((threadIdx.x & 31) == 0 && !sched_aborted(s)) t = static_cast<int>(atomicAdd(s.counter, 1u));
+    t = __shfl_sync(0xffffffffu, t, 0);
+    if (t < 0 || t >= s.total) return false;
     const SchedTile d = decode_ticket(s, t);
     if (!sched_wait(s, d)) return false;
-    *out = d;
+    if ((threadIdx.x & 31) == 0) *out = d;
     return true;
 }
 
