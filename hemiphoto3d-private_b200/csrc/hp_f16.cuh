@@ -108,18 +108,18 @@ struct RefStats {
 // Shared memory of a CTA (dynamic: the widest windows pass the 48 KB static
 // limit).  Windows kept in s_win need the reference tile only while they are
 // built, so the half-pass's source costs then take its place.
-template <int R, int ST, int TH>
+template <int R, int ST, int TH, int THREADS = 32 * TH>
 struct alignas(16) Shared {
-    static constexpr int NT = 32 * TH;
+    static constexpr int NT = THREADS, PX = 32 * TH;  // threads, active pixels of a half-pass
     static constexpr int REF = (TILE_W + 2 * R) * (TH + 2 * R);
     static constexpr int UNITS = HP_MAX_SOURCES * NT;
     static constexpr bool OVERLAY = Win<R, ST>::IN_SMEM;
-    __half2 win[OVERLAY ? Win<R, ST>::SIDE * Win<R, ST>::VEC * NT : 4];  // see load_window
+    __half2 win[OVERLAY ? Win<R, ST>::SIDE * Win<R, ST>::VEC * PX : 4];  // see load_window
     float4 plane[NT];               // half-pass: plane_vector of the chunk's items
     float ref[OVERLAY ? (REF > UNITS ? REF : UNITS) : REF];
     float unit_own[OVERLAY ? 1 : UNITS];
-    float2 stat[NT];                // half-pass: (mean, ssd) of each thread's pixel window
-    PassShared<NT> pass;
+    float2 stat[PX];                // half-pass: (mean, ssd) of each pixel's window
+    PassShared<NT, PX> pass;
     __device__ __forceinline__ float* units() { return OVERLAY ? ref : unit_own; }  // half-pass: source costs
 };
 
@@ -578,9 +578,9 @@ __device__ __forceinline__ float unit_cost(const ViewDesc* __restrict__ v, int s
 }
 
 extern __shared__ __align__(16) unsigned char dynamic_smem[];
-template <int R, int ST, int TH>
-__device__ __forceinline__ Shared<R, ST, TH>& shared_of() {
-    return *reinterpret_cast<Shared<R, ST, TH>*>(dynamic_smem);
+template <int R, int ST, int TH, int NT = 32 * TH>
+__device__ __forceinline__ Shared<R, ST, TH, NT>& shared_of() {
+    return *reinterpret_cast<Shared<R, ST, TH, NT>*>(dynamic_smem);
 }
 
 template <int R, int ST, int TH, int D>
@@ -624,17 +624,19 @@ __global__ void __launch_bounds__(Tile<TH>::NT, Tile<TH>::MIN_BLOCKS) cost16_ker
 
 // Scorer of the half-pass (red_black_pass): a unit reads its pixel's window
 // statistics and s_win column, and its item's plane vector, from shared memory.
-template <int R, int ST, int TH, int D>
+template <int R, int ST, int TH, int D, int NT>
 struct Scorer16 {
-    static constexpr int NT = Tile<TH>::NT, TW = TILE_W + 2 * R;
+    static constexpr int PX = 32 * TH, TW = TILE_W + 2 * R;
     static constexpr bool BLOCKS = !Win<R, ST>::IN_SMEM, BY_PLANE = false, WHOLE_WARPS = false;
     const ViewDesc* v;
-    Shared<R, ST, TH>& sm;
+    Shared<R, ST, TH, NT>& sm;
     int x0, y0;
     unsigned soft_mask;
     RefStats st{0.f, 0.f};
-    __device__ __forceinline__ void begin(int lx, int ly) { st = load_window<R, ST, NT>(sm.win, sm.ref, TW, lx, ly); }
-    __device__ __forceinline__ void publish() { sm.stat[threadIdx.x] = make_float2(st.mean, st.ssd); }
+    __device__ __forceinline__ void begin(int lx, int ly) { st = load_window<R, ST, PX>(sm.win, sm.ref, TW, lx, ly); }
+    __device__ __forceinline__ void publish() {
+        if (NT == PX || threadIdx.x < PX) sm.stat[threadIdx.x] = make_float2(st.mean, st.ssd);
+    }
     __device__ __forceinline__ void set_plane(int k, int x, int y, float4 h, bool ok) {
         sm.plane[k] = ok ? plane_vector(v, x, y, h) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
@@ -642,29 +644,32 @@ struct Scorer16 {
         const float2 os = sm.stat[o];
         const float4 m = sm.plane[k];
         if (m.w == 0.0f) return 2.0f;
-        return unit_cost<R, ST, NT, D>(v, s, m.x, m.y, m.z, RefStats{os.x, os.y}, sm.win + o * Win<R, ST>::VEC,
+        return unit_cost<R, ST, PX, D>(v, s, m.x, m.y, m.z, RefStats{os.x, os.y}, sm.win + o * Win<R, ST>::VEC,
                                        sm.ref, TW, lx, ly, x0 + lx, y0 + ly, soft_mask);
     }
     __device__ __forceinline__ float mean(float sum, int k) const { return __fdiv_rn(sum, static_cast<float>(k)); }
 };
 
-template <int R, int ST, int TH, int D>
-__device__ __forceinline__ void tile_propagate16(const ViewDesc* v, int tile_x, int tile_y, const SolveConsts& sc,
-                                                 int iteration, int color, Shared<R, ST, TH>& sm) {
-    constexpr int NT = Tile<TH>::NT;
-    const int x0 = tile_x * TILE_W, y0 = tile_y * TH;
+template <int R, int ST, int TH, int D, int NT>
+__device__ __forceinline__ void tile_propagate16(const ViewDesc* v, int x0, int y0, const SolveConsts& sc,
+                                                 int iteration, int color, Shared<R, ST, TH, NT>& sm,
+                                                 bool roomy = false) {
     load_ref_tile16<NT>(sm.ref, TILE_W + 2 * R, TH + 2 * R, v, x0, y0, R);
     __syncthreads();
-    Scorer16<R, ST, TH, D> scorer{v, sm, x0, y0, sc.soft_mask};
-    red_black_pass<NT>(v, x0, y0, sc, iteration, color, scorer, sm.units(), sm.pass);
+    Scorer16<R, ST, TH, D, NT> scorer{v, sm, x0, y0, sc.soft_mask};
+    red_black_pass<NT, 32 * TH>(v, x0, y0, sc, iteration, color, scorer, sm.units(), sm.pass, roomy);
 }
 
-template <int R, int ST, int TH, int D>
+// SPLIT: two CTAs of half the tile's rows and all its threads to a tile (split_tiles).
+template <int R, int ST, int TH, int D, bool SPLIT>
 __global__ void __launch_bounds__(Tile<TH>::NT, Tile<TH>::MIN_BLOCKS) propagate16_kernel(BatchList bl, SolveConsts sc,
-                                                                                       int iteration, int color) {
+                                                                                       int iteration, int color,
+                                                                                       bool roomy) {
+    constexpr int ROWS = SPLIT ? TH / 2 : TH, NT = Tile<TH>::NT;
     int tile_x, tile_y;
-    const ViewDesc* v = locate_tile16(bl, blockIdx.x, &tile_x, &tile_y);
-    tile_propagate16<R, ST, TH, D>(v, tile_x, tile_y, sc, iteration, color, shared_of<R, ST, TH>());
+    const ViewDesc* v = locate_tile16(bl, SPLIT ? blockIdx.x >> 1 : blockIdx.x, &tile_x, &tile_y);
+    tile_propagate16<R, ST, ROWS, D, NT>(v, tile_x * TILE_W, tile_y * TH + (SPLIT ? (blockIdx.x & 1) * ROWS : 0), sc,
+                                         iteration, color, shared_of<R, ST, ROWS, NT>(), roomy);
 }
 
 // Persistent form (see Schedule and the FP32 persistent kernel): the stage
@@ -708,7 +713,7 @@ __global__ void __launch_bounds__(Tile<TH>::NT, Tile<TH>::MIN_BLOCKS) persistent
             tile_cost16<R, ST, TH, D>(v, tx, ty, s.sc, sm);
         } else if (stage <= 2 * v->iterations) {
             const int k = stage - 1;
-            tile_propagate16<R, ST, TH, D>(v, tx, ty, s.sc, k >> 1, k & 1, sm);
+            tile_propagate16<R, ST, TH, D, Tile<TH>::NT>(v, tx * TILE_W, ty * TH, s.sc, k >> 1, k & 1, sm);
         } else if (is_filter_stage(v, stage)) {
             tile_filter(s.views, v, tx, ty, true);  // geometric check, then the maps
         } else {
@@ -745,8 +750,21 @@ struct Dispatch {
             if ((e = allow(reinterpret_cast<const void*>(cost16_kernel<R, ST, TH, D>))) != cudaSuccess) return e;
             cost16_kernel<R, ST, TH, D><<<bl->total_tiles, NT, smem, st>>>(*bl, sc);
         } else {
-            if ((e = allow(reinterpret_cast<const void*>(propagate16_kernel<R, ST, TH, D>))) != cudaSuccess) return e;
-            propagate16_kernel<R, ST, TH, D><<<bl->total_tiles, NT, smem, st>>>(*bl, sc, iteration, color);
+            if constexpr (TH == 8) {
+                const int sms = device_sms();
+                if (split_tiles(bl->total_tiles, sms)) {  // 4 loads in flight: the staging depth changes no bit
+                    constexpr int half = static_cast<int>(sizeof(Shared<R, ST, TH / 2, NT>));
+                    if ((e = cudaFuncSetAttribute(propagate16_kernel<R, ST, TH, 4, true>,
+                                                  cudaFuncAttributeMaxDynamicSharedMemorySize, half)) != cudaSuccess)
+                        return e;
+                    propagate16_kernel<R, ST, TH, 4, true><<<2 * bl->total_tiles, NT, half, st>>>(
+                        *bl, sc, iteration, color, 2 * bl->total_tiles <= 3 * sms);
+                    return cudaGetLastError();
+                }
+            }
+            if ((e = allow(reinterpret_cast<const void*>(propagate16_kernel<R, ST, TH, D, false>))) != cudaSuccess)
+                return e;
+            propagate16_kernel<R, ST, TH, D, false><<<bl->total_tiles, NT, smem, st>>>(*bl, sc, iteration, color, false);
         }
         return cudaGetLastError();
     }

@@ -85,6 +85,29 @@ struct SolveConsts {
     int memo;            // half-passes keep and use the settled bit of stored costs (whole solves: 1)
 };
 
+// Small per-pass launches can run two CTAs on each 64 x 8 tile, 64 x 4 pixels
+// with the same 256 threads.  That pays
+//  - up to one tile an SM: a GPU that is not full gets twice the warps, and each
+//    takes half as many turns of (item, source) units;
+//  - beyond, when half tiles spread better: the busiest SM's share is
+//    ceil(2 t / SMs) halves instead of 2 ceil(t / SMs), less when the part of
+//    t / SMs past its whole number lies in (0, 1/2].  Past 8 tiles an SM there is
+//    little left to gain.
+// Measured, whole tiles -> halves (148 SMs): FP16-acc r 7 s 2, 4 sources, 8
+// iterations, 320 x 240 (150 tiles) 1914 -> 1540 us, 480 x 360 (360) 2708 ->
+// 2385, 560 x 420 (477) 3119 -> 2915, but 400 x 300 (266) 1965 -> 2006 and 720 x
+// 540 (816) 4210 -> 4254; FP32 r 5 s 1, 320 x 240, 2 sources, 4 iterations 1154
+// -> 975 us, 480 x 360, 6 sources 7353 -> 6703, 400 x 300 3779 -> 4007.
+inline bool split_tiles(int tiles, int sms) {
+    const int past = tiles % sms;
+    return tiles <= sms || (tiles <= 8 * sms && past > 0 && 2 * past <= sms);
+}
+inline int device_sms() {
+    int dev = 0, sms = 148;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms;
+}
+
 // A batch launch covers the tiles of several views: view k owns flattened
 // tile indices [tile_prefix[k], tile_prefix[k+1]).
 struct BatchList {

@@ -49,9 +49,6 @@ template <int R, int ST>
 constexpr int pass_blocks() { return (2 * R) / ST + 1 <= 8 ? 4 : 3; }
 constexpr int COST_BLOCKS = 3;  // full-map cost, 1920 x 1080, r 5, s 1: 1486 us, 1574 with 2, 1506 with 4
 
-constexpr int MAX_TW = TILE_W + 2 * HP_MAX_RADIUS;
-constexpr int MAX_TH = TILE_H + 2 * HP_MAX_RADIUS;
-
 // Locate the view and tile of this CTA in a batch launch.
 __device__ __forceinline__ const ViewDesc* locate_tile(const BatchList& bl, int t, int* tx, int* ty) {
     int lo = 0, hi = bl.n_active - 1;
@@ -324,22 +321,21 @@ __device__ __forceinline__ float mean_f32(float sum, int k) { return sum / stati
 
 // Full-map cost of the current hypotheses of one tile (compute_ncc_cost_kernel,
 // patchmatch_mvs.cu:349-513).  Each thread owns two pixels of its row.
-template <int R, int ST>
-__device__ __forceinline__ void tile_cost(const ViewDesc* v, int tile_x, int tile_y, const SolveConsts& sc,
-                                          float* s_ref) {
-    constexpr int tw = TILE_W + 2 * R, th = TILE_H + 2 * R;
-    const int x0 = tile_x * TILE_W, y0 = tile_y * TILE_H;
+template <int R, int ST, int TH>
+__device__ __forceinline__ void tile_cost(const ViewDesc* v, int x0, int y0, const SolveConsts& sc, float* s_ref) {
+    constexpr int tw = TILE_W + 2 * R, th = TH + 2 * R;
     load_ref_tile(s_ref, tw, th, v, x0, y0, R);
     __syncthreads();
-    const int ly = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int y = y0 + ly;
+    // Lanes own consecutive pixels (a warp 32 of a tile row): its taps of one
+    // window position then lie next to each other.
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    constexpr int WARPS_A_ROW = CTA_THREADS / 32 / TH;  // 1, each taking both halves of its row, or 2
+    const int ly = warp / WARPS_A_ROW, y = y0 + ly;
     if (y >= v->H) return;
-    // Lanes own consecutive pixels (two 32-pixel halves of the tile row): a
-    // warp's taps of one window position then lie next to each other.
-    for (int j = 0; j < 2; ++j) {
+    for (int j = 0; j < 2 / WARPS_A_ROW; ++j) {
         // Whole warps score; lanes past the image repeat its last column.
-        const int lx = min(32 * j + lane, v->W - 1 - x0), x = x0 + lx;
-        if (lx < 32 * j) break;
+        const int left = 32 * (j + warp % WARPS_A_ROW), lx = min(left + lane, v->W - 1 - x0), x = x0 + lx;
+        if (lx < left) break;
         const size_t idx = static_cast<size_t>(y) * v->W + x;
         const PlaneF32 p = plane_f32(v, x, y, v->hyp[idx]);
         const float2 sums = window_sums<R, ST>(s_ref, tw, lx, ly);
@@ -349,30 +345,33 @@ __device__ __forceinline__ void tile_cost(const ViewDesc* v, int tile_x, int til
     }
 }
 
-template <int R, int ST>
+// SPLIT: two CTAs of 64 x 4 pixels to a tile (split_tiles).
+template <int R, int ST, bool SPLIT>
 __global__ void __launch_bounds__(CTA_THREADS, COST_BLOCKS) cost_kernel(BatchList bl, SolveConsts sc) {
-    __shared__ float s_ref[MAX_TW * MAX_TH];
+    constexpr int TH = SPLIT ? TILE_H / 2 : TILE_H;
+    __shared__ float s_ref[(TILE_W + 2 * R) * (TH + 2 * R)];
     int tile_x, tile_y;
-    const ViewDesc* v = locate_tile(bl, blockIdx.x, &tile_x, &tile_y);
-    tile_cost<R, ST>(v, tile_x, tile_y, sc, s_ref);
+    const ViewDesc* v = locate_tile(bl, SPLIT ? blockIdx.x >> 1 : blockIdx.x, &tile_x, &tile_y);
+    tile_cost<R, ST, TH>(v, tile_x * TILE_W, tile_y * TILE_H + (SPLIT ? (blockIdx.x & 1) * TH : 0), sc, s_ref);
 }
 
 // Shared memory of a half-pass beyond the reference tile.
+template <int PX>
 struct Shared32 {
     float4 plane[CTA_THREADS];  // nK and 1 / (n.P) of the chunk's items
     float unit[HP_MAX_SOURCES * CTA_THREADS];
     unsigned char ok[CTA_THREADS];
-    float2 sums[CTA_THREADS];   // window_sums of each thread's pixel
-    PassShared<CTA_THREADS> pass;
+    float2 sums[PX];            // window_sums of each pixel
+    PassShared<CTA_THREADS, PX> pass;
 };
 
 // Scorer of the half-pass (red_black_pass).
-template <int R, int ST>
+template <int R, int ST, int PX>
 struct Scorer32 {
     static constexpr bool BLOCKS = true, BY_PLANE = true, WHOLE_WARPS = true;
     const ViewDesc* v;
     const float* s_ref;
-    Shared32& sm;
+    Shared32<PX>& sm;
     int x0, y0;
     __device__ __forceinline__ void begin(int lx, int ly) {
         sm.sums[threadIdx.x] = window_sums<R, ST>(s_ref, TILE_W + 2 * R, lx, ly);
@@ -391,25 +390,28 @@ struct Scorer32 {
     __device__ __forceinline__ float mean(float sum, int k) const { return mean_f32(sum, k); }
 };
 
-template <int R, int ST>
-__device__ __forceinline__ void tile_propagate(const ViewDesc* v, int tile_x, int tile_y, const SolveConsts& sc,
-                                               int iteration, int color, float* s_ref, Shared32& sm) {
-    const int x0 = tile_x * TILE_W, y0 = tile_y * TILE_H;
-    load_ref_tile(s_ref, TILE_W + 2 * R, TILE_H + 2 * R, v, x0, y0, R);
+template <int R, int ST, int TH>
+__device__ __forceinline__ void tile_propagate(const ViewDesc* v, int x0, int y0, const SolveConsts& sc,
+                                               int iteration, int color, float* s_ref, Shared32<TILE_W * TH / 2>& sm,
+                                               bool roomy = false) {
+    constexpr int PX = TILE_W * TH / 2;
+    load_ref_tile(s_ref, TILE_W + 2 * R, TH + 2 * R, v, x0, y0, R);
     __syncthreads();
-    Scorer32<R, ST> scorer{v, s_ref, sm, x0, y0};
-    red_black_pass<CTA_THREADS>(v, x0, y0, sc, iteration, color, scorer, sm.unit, sm.pass);
+    Scorer32<R, ST, PX> scorer{v, s_ref, sm, x0, y0};
+    red_black_pass<CTA_THREADS, PX>(v, x0, y0, sc, iteration, color, scorer, sm.unit, sm.pass, roomy);
 }
 
-template <int R, int ST>
+template <int R, int ST, bool SPLIT>
 __global__ void __launch_bounds__(CTA_THREADS, pass_blocks<R, ST>()) propagate_kernel(BatchList bl,
                                                                                          SolveConsts sc, int iteration,
-                                                                                         int color) {
-    __shared__ float s_ref[MAX_TW * MAX_TH];
-    __shared__ Shared32 sm;
+                                                                                         int color, bool roomy) {
+    constexpr int TH = SPLIT ? TILE_H / 2 : TILE_H;
+    __shared__ float s_ref[(TILE_W + 2 * R) * (TH + 2 * R)];
+    __shared__ Shared32<TILE_W * TH / 2> sm;
     int tile_x, tile_y;
-    const ViewDesc* v = locate_tile(bl, blockIdx.x, &tile_x, &tile_y);
-    tile_propagate<R, ST>(v, tile_x, tile_y, sc, iteration, color, s_ref, sm);
+    const ViewDesc* v = locate_tile(bl, SPLIT ? blockIdx.x >> 1 : blockIdx.x, &tile_x, &tile_y);
+    const int y0 = tile_y * TILE_H + (SPLIT ? (blockIdx.x & 1) * TH : 0);
+    tile_propagate<R, ST, TH>(v, tile_x * TILE_W, y0, sc, iteration, color, s_ref, sm, roomy);
 }
 
 // Persistent form: one launch runs every stage of every view of a solve
@@ -418,8 +420,8 @@ __global__ void __launch_bounds__(CTA_THREADS, pass_blocks<R, ST>()) propagate_k
 // are bit-identical to the per-stage launch sequence.
 template <int R, int ST>
 __global__ void __launch_bounds__(CTA_THREADS, pass_blocks<R, ST>()) persistent_kernel(Schedule s) {
-    __shared__ float s_ref[MAX_TW * MAX_TH];
-    __shared__ Shared32 sm;
+    __shared__ float s_ref[(TILE_W + 2 * R) * (TILE_H + 2 * R)];
+    __shared__ Shared32<CTA_THREADS> sm;
     // The claimed tile lives in shared memory: warp 0 decodes it once and
     // thread 0 publishes it after the stage, so no thread carries it through the body.
     __shared__ SchedTile s_tile;
@@ -439,10 +441,10 @@ __global__ void __launch_bounds__(CTA_THREADS, pass_blocks<R, ST>()) persistent_
         if (stage == 0) {
             tile_init(v, tx, ty);
             __syncthreads();
-            tile_cost<R, ST>(v, tx, ty, s.sc, s_ref);
+            tile_cost<R, ST, TILE_H>(v, tx * TILE_W, ty * TILE_H, s.sc, s_ref);
         } else if (stage <= 2 * v->iterations) {
             const int k = stage - 1;
-            tile_propagate<R, ST>(v, tx, ty, s.sc, k >> 1, k & 1, s_ref, sm);
+            tile_propagate<R, ST, TILE_H>(v, tx * TILE_W, ty * TILE_H, s.sc, k >> 1, k & 1, s_ref, sm);
         } else if (is_filter_stage(v, stage)) {
             tile_filter(s.views, v, tx, ty, true);  // geometric check, then the maps
         } else {
@@ -456,10 +458,17 @@ __global__ void __launch_bounds__(CTA_THREADS, pass_blocks<R, ST>()) persistent_
 template <int R, int ST>
 cudaError_t launch_rs(const BatchList& bl, const SolveConsts& sc, int iteration, int color, bool full,
                       cudaStream_t st) {
-    if (full)
-        cost_kernel<R, ST><<<bl.total_tiles, CTA_THREADS, 0, st>>>(bl, sc);
-    else
-        propagate_kernel<R, ST><<<bl.total_tiles, CTA_THREADS, 0, st>>>(bl, sc, iteration, color);
+    const int tiles = bl.total_tiles, sms = device_sms();
+    if (split_tiles(tiles, sms)) {
+        if (full)
+            cost_kernel<R, ST, true><<<2 * tiles, CTA_THREADS, 0, st>>>(bl, sc);
+        else
+            propagate_kernel<R, ST, true><<<2 * tiles, CTA_THREADS, 0, st>>>(bl, sc, iteration, color, 2 * tiles <= 3 * sms);
+    } else if (full) {
+        cost_kernel<R, ST, false><<<tiles, CTA_THREADS, 0, st>>>(bl, sc);
+    } else {
+        propagate_kernel<R, ST, false><<<tiles, CTA_THREADS, 0, st>>>(bl, sc, iteration, color, false);
+    }
     return cudaGetLastError();
 }
 

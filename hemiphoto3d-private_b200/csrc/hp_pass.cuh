@@ -56,14 +56,14 @@ struct Lowest {
     }
 };
 
-// Shared memory of a half-pass with NT threads, beyond the scorer's own and the
-// source costs (HP_MAX_SOURCES rows of NT floats: cost of item k at the q-th
-// source of the view's order at q * NT + k).
-template <int NT>
+// Shared memory of a half-pass with NT threads on PX active pixels, beyond the
+// scorer's own and the source costs (HP_MAX_SOURCES rows of NT floats: cost of
+// item k at the q-th source of the view's order at q * NT + k).
+template <int NT, int PX>
 struct PassShared {
-    float cost[NT * 4];            // neighbour costs, slot (thread << 2 | cand)
-    unsigned short items[NT * 4];  // neighbour items (thread << 2 | cand), then the surviving trials
-    unsigned char need[NT];        // neighbour planes each thread's pixel scores (bit per cand)
+    float cost[PX * 4];            // neighbour costs, slot (thread << 2 | cand)
+    unsigned short items[PX * 4];  // neighbour items (thread << 2 | cand), then the surviving trials
+    unsigned char need[PX];        // neighbour planes each thread's pixel scores (bit per cand)
     int warp_total[NT / 32];
     int survivors;
 };
@@ -95,8 +95,10 @@ __device__ __forceinline__ int pass_thread(int lx, int ly) {
                   : ly << 5 | lx >> 1;
 }
 
-// One half-pass of the tile at (x0, y0), TILE_W x NT / 32 pixels: every thread
-// owns an active pixel, where the reference idles half its grid.
+// One half-pass of the tile at (x0, y0), TILE_W x PX / 32 pixels: threads below
+// PX own an active pixel each, where the reference idles half its grid.  The
+// others, in launches of half tiles (split_tiles), only score.  `roomy`: the
+// launch leaves SMs with idle warps.
 // The scorer K, per thread:
 //   begin(lx, ly)               prepares the window of the thread's own pixel (active pixels only)
 //   publish()                   makes it readable by the other threads (after the next barrier)
@@ -106,17 +108,17 @@ __device__ __forceinline__ int pass_thread(int lx, int ly) {
 //   BLOCKS                      pass_pixel's layout
 //   BY_PLANE                    neighbour items are listed by the plane they score, not by pixel
 //   WHOLE_WARPS                 score needs all 32 lanes of a warp together
-template <int NT, class K>
+template <int NT, int PX, class K>
 __device__ __forceinline__ void red_black_pass(const ViewDesc* v, int x0, int y0, const SolveConsts& sc,
                                                int iteration, int color, K& scorer, float* unit,
-                                               PassShared<NT>& sm) {
+                                               PassShared<NT, PX>& sm, bool roomy = false) {
     const int W = v->W, H = v->H, S = v->S;
     const int tid = threadIdx.x, lane = tid & 31;
     const int2 own = pass_pixel<K::BLOCKS>(tid, y0, color);
     const int lx = own.x, ly = own.y, x = x0 + lx, y = y0 + ly;
     // Read through a broadcast: the compiler then knows that it is the same for a warp's lanes.
     const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
-    const bool active = y < H && x < W;  // every thread takes part in the barriers
+    const bool active = (NT == PX || tid < PX) && y < H && x < W;  // every thread takes part in the barriers
     const size_t idx = static_cast<size_t>(y) * W + x;
     float4 best = make_float4(0.f, 0.f, 0.f, 0.f);
     float best_cost = 0.f;
@@ -141,13 +143,13 @@ __device__ __forceinline__ void red_black_pass(const ViewDesc* v, int x0, int y0
         return pass_thread<K::BLOCKS>(nx + (c == 0 ? 1 : (c == 1 ? -1 : 0)), ny + (c == 2 ? 1 : (c == 3 ? -1 : 0)));
     };
     if constexpr (K::BY_PLANE) {
-        sm.need[tid] = static_cast<unsigned char>(need);
+        if (NT == PX || tid < PX) sm.need[tid] = static_cast<unsigned char>(need);
         __syncthreads();
         list = 0;
-        constexpr int TH = NT / 32;
+        constexpr int TH = PX / 32;
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-            const bool in = c == 0 ? nx + 1 < TILE_W : (c == 1 ? nx > 0 : (c == 2 ? ny + 1 < TH : ny > 0));
+            const bool in = (NT == PX || tid < PX) && (c == 0 ? nx + 1 < TILE_W : (c == 1 ? nx > 0 : (c == 2 ? ny + 1 < TH : ny > 0)));
             if (in && ((sm.need[owner(c)] >> c) & 1u)) list |= 1u << c;
             const bool outside = c == 0 ? lx == 0 : (c == 1 ? lx + 1 == TILE_W : (c == 2 ? ly == 0 : ly + 1 == TH));
             if (outside && ((need >> c) & 1u)) list |= 16u << c;
@@ -182,7 +184,9 @@ __device__ __forceinline__ void red_black_pass(const ViewDesc* v, int x0, int y0
     // in them, and a texture handle stays in a uniform register (with a scorer's votes inside it is otherwise fetched
     // lane by lane: FP32, 2 x 1920 x 1080, 149.7 ms against 115.1).
     total = __shfl_sync(0xffffffffu, total, 0);
-    const int kk = min(sc.top_k, S), lead = S - kk + 1;
+    const int kk = min(sc.top_k, S);
+    // With warps idle, two parts of few sources would take two turns where one takes one.
+    const int lead = roomy && S <= 3 ? S : S - kk + 1;
     float drange = __fmul_rn(__fsub_rn(v->dmax, v->dmin), 0.5f);
     float nrange = 1.0f;
     for (int i = 0; i < iteration; ++i) {
@@ -210,7 +214,7 @@ __device__ __forceinline__ void red_black_pass(const ViewDesc* v, int x0, int y0
             drange = __fmul_rn(drange, sc.step_decay);
             nrange = __fmul_rn(nrange, sc.step_decay);
         }
-        const int count = round == 0 ? total : NT;
+        const int count = round == 0 ? total : PX;
         float c = 2.0f;
         bool keep = true;
 #pragma unroll 1
