@@ -765,9 +765,9 @@ def run_serving(args, hp, device: int):
 
 
 def run_count_taps(args):
-    """Executed taps: the instrumented engine counts, per sampled (candidate, source), its window's taps
-    (wholly-outside sources and duplicate neighbour planes are skipped, as in the timed kernels).  Views 0 and
-    10 of the headline workload are solved pass by pass (hp_propagate_pass), so only the half-passes count."""
+    """Executed taps: the instrumented engine counts, per sampled (candidate, source), its window's taps.  Views 0
+    and 10 of the headline workload are solved with 0, 1, 2, ... iterations; the difference between two solves is
+    an iteration's taps (single half-passes, hp_propagate_pass, leave out less than a solve does)."""
     import ctypes as C
     hp = importlib.import_module(PKG)
     L = C.CDLL(hp.LIB_PATH)
@@ -787,14 +787,16 @@ def run_count_taps(args):
                                   *WORKLOAD["depth_range"], seed=42, view_id=r, iterations=WORKLOAD["iterations"])
                 p = hp.default_params(radius=WORKLOAD["radius"], stride=WORKLOAD["stride"], precision=prec)
                 m, _, _, _ = hp.host_maps(s.height, s.width)
-                ctx.init_hypotheses(job, p, m)
-                ctx.ncc_cost(job, p, m)
                 L.hp_debug_taps(C.byref(f32c), C.byref(f16c))
-                for it in range(WORKLOAD["iterations"]):
-                    for color in (0, 1):
-                        ctx.propagate_pass(job, p, m, it, color)
+                before = 0
+                for it in range(WORKLOAD["iterations"] + 1):
+                    job.iterations = it
+                    ctx.solve([job], p, [m])
                     L.hp_debug_taps(C.byref(f32c), C.byref(f16c))
-                    per_it[it] += (f32c if name == "f32" else f16c).value
+                    taps = (f32c if name == "f32" else f16c).value
+                    if it > 0:
+                        per_it[it - 1] += taps - before
+                    before = taps
             visits_per_it = len(refs) * s.height * s.width  # two half-passes of W * H / 2 visits per view
             out[name] = {"executed_taps_per_pixel_visit": round(float(per_it.sum() / (visits_per_it * len(per_it))), 1),
                          "per_iteration": [round(float(x / visits_per_it), 1) for x in per_it],

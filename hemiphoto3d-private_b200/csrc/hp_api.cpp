@@ -543,6 +543,7 @@ hp_status hp_ctx_destroy(hp_ctx* ctx) {
         ctx->descs.release();
         ctx->lists.release();
         ctx->staging.release();
+        ctx->fuse.release();
         ctx->seedbuf.release();
         ctx->filters.release();
         for (cudaEvent_t e : ctx->events) cudaEventDestroy(e);
@@ -921,7 +922,7 @@ hp_status hp_fuse_depth_maps(hp_ctx* ctx, const hp_fuse_view* views, int num_vie
         return fail(ctx, HP_ERR_INVALID_ARG, "fuse: tolerance out of range");
     if (out->capacity < 0) return fail(ctx, HP_ERR_INVALID_ARG, "fuse: negative capacity");
     DeviceGuard g(ctx->device);
-    // Device scratch freed on every return path (cudaFree waits for the device).
+    // Device memory of a host cloud, freed on every return path (cudaFree waits for the device).
     struct Scratch {
         void* p = nullptr;
         ~Scratch() {
@@ -931,8 +932,11 @@ hp_status hp_fuse_depth_maps(hp_ctx* ctx, const hp_fuse_view* views, int num_vie
     const bool dev_in = prm->memory == HP_MEMORY_DEVICE;
     std::vector<hp::FuseView> fv(num_views);
     std::vector<int> nbs, vblock(num_views + 1);
-    long long blocks = 0;
+    long long blocks = 0, pixels = 0;
     size_t staged_floats = 0;
+    for (int i = 0; i < num_views; ++i)
+        if (views[i].width > 0 && views[i].height > 0) pixels += static_cast<long long>(views[i].width) * views[i].height;
+    const int steps = hp::fuse_steps(pixels), cta_px = steps * hp::FUSE_THREADS;
     for (int i = 0; i < num_views; ++i) {
         const hp_fuse_view& v = views[i];
         if (v.width < 1 || v.height < 1 || v.width > 65536 || v.height > 65536)
@@ -966,7 +970,7 @@ hp_status hp_fuse_depth_maps(hp_ctx* ctx, const hp_fuse_view* views, int num_vie
         f.nb_count = static_cast<int>(nbs.size()) - f.nb_begin;
         vblock[i] = static_cast<int>(blocks);
         const size_t px = static_cast<size_t>(v.width) * v.height;
-        blocks += static_cast<long long>((px + hp::FUSE_PIXELS - 1) / hp::FUSE_PIXELS);
+        blocks += static_cast<long long>((px + cta_px - 1) / cta_px);
         // The one-CTA scan indexes the per-CTA counts with ints; 2^28 CTAs (2.7e11 pixels) keep them in range.
         if (blocks > (1ll << 28)) return fail(ctx, HP_ERR_INVALID_ARG, "fuse: too many pixels");
         staged_floats += px * (4 + (v.confidence ? 1 : 0) + (v.gray ? 1 : 0));
@@ -1003,23 +1007,22 @@ hp_status hp_fuse_depth_maps(hp_ctx* ctx, const hp_fuse_view* views, int num_vie
     const size_t o_nb = up8(sizeof(hp::FuseView) * num_views);
     const size_t o_vb = o_nb + up8(sizeof(int) * std::max<size_t>(nbs.size(), 1));
     const size_t o_bal = o_vb + up8(sizeof(int) * (num_views + 1));
-    const size_t o_cnt = o_bal + sizeof(unsigned) * (hp::FUSE_PIXELS / 32) * blocks;
+    const size_t o_cnt = o_bal + up8(sizeof(unsigned) * (cta_px / 32) * blocks);
     const size_t o_off = o_cnt + up8(sizeof(int) * blocks);
     const size_t o_tot = o_off + sizeof(long long) * blocks;
-    Scratch desc;
-    HP_CUDA(cudaMalloc(&desc.p, o_tot + sizeof(long long)));
-    char* base = static_cast<char*>(desc.p);
-    HP_CUDA(cudaMemcpyAsync(base, fv.data(), sizeof(hp::FuseView) * num_views, cudaMemcpyHostToDevice, ctx->stream));
-    if (!nbs.empty())
-        HP_CUDA(cudaMemcpyAsync(base + o_nb, nbs.data(), sizeof(int) * nbs.size(), cudaMemcpyHostToDevice,
-                                ctx->stream));
-    HP_CUDA(cudaMemcpyAsync(base + o_vb, vblock.data(), sizeof(int) * (num_views + 1), cudaMemcpyHostToDevice,
-                            ctx->stream));
+    HP_CUDA(ctx->fuse.ensure(o_tot + sizeof(long long)));
+    char* base = static_cast<char*>(ctx->fuse.p);
+    std::vector<char> up(o_bal);  // views, neighbours and first CTAs in one copy
+    std::memcpy(up.data(), fv.data(), sizeof(hp::FuseView) * num_views);
+    if (!nbs.empty()) std::memcpy(up.data() + o_nb, nbs.data(), sizeof(int) * nbs.size());
+    std::memcpy(up.data() + o_vb, vblock.data(), sizeof(int) * (num_views + 1));
+    HP_CUDA(cudaMemcpyAsync(base, up.data(), up.size(), cudaMemcpyHostToDevice, ctx->stream));
     hp::FuseArgs a;
     a.views = reinterpret_cast<const hp::FuseView*>(base);
     a.neighbors = reinterpret_cast<const int*>(base + o_nb);
     a.view_block = reinterpret_cast<const int*>(base + o_vb);
     a.n_views = num_views;
+    a.steps = steps;
     a.min_views = prm->min_views;
     a.min_conf = prm->min_confidence;
     a.max_depth_rel = prm->max_depth_rel;

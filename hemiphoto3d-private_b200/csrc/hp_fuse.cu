@@ -196,8 +196,7 @@ __device__ __forceinline__ Fused fuse_pixel(const FuseArgs& a, int i, int x, int
     return f;
 }
 
-constexpr int FUSE_STEPS = FUSE_PIXELS / FUSE_THREADS;
-constexpr int FUSE_WORDS = FUSE_PIXELS / 32;  // ballot words per CTA
+constexpr int STEP_WORDS = FUSE_THREADS / 32;  // ballot words per step
 constexpr int FUSE_BLOCKS = 6;                // resident CTAs per SM the passes are register-budgeted for
 
 __global__ void __launch_bounds__(FUSE_THREADS, FUSE_BLOCKS) fuse_count_kernel(FuseArgs a, unsigned* ballots,
@@ -205,10 +204,11 @@ __global__ void __launch_bounds__(FUSE_THREADS, FUSE_BLOCKS) fuse_count_kernel(F
     const int i = fuse_view_of(a, blockIdx.x);
     const int W = a.views[i].W;
     const long long px = static_cast<long long>(W) * a.views[i].H;
-    const long long first = static_cast<long long>(blockIdx.x - a.view_block[i]) * FUSE_PIXELS + threadIdx.x;
+    const long long first = static_cast<long long>(blockIdx.x - a.view_block[i]) * a.steps * FUSE_THREADS +
+                            threadIdx.x;
     int n = 0;
 #pragma unroll 1
-    for (int step = 0; step < FUSE_STEPS; ++step) {
+    for (int step = 0; step < a.steps; ++step) {
         const long long p = first + step * FUSE_THREADS;
         bool emit = false;
         if (p < px) {
@@ -217,8 +217,7 @@ __global__ void __launch_bounds__(FUSE_THREADS, FUSE_BLOCKS) fuse_count_kernel(F
         }
         const unsigned votes = __ballot_sync(0xffffffffu, emit);
         if ((threadIdx.x & 31) == 0)
-            ballots[static_cast<size_t>(blockIdx.x) * FUSE_WORDS + step * (FUSE_THREADS / 32) + (threadIdx.x >> 5)] =
-                votes;
+            ballots[(static_cast<size_t>(blockIdx.x) * a.steps + step) * STEP_WORDS + (threadIdx.x >> 5)] = votes;
         n += emit;
     }
     __shared__ int total;
@@ -281,12 +280,14 @@ __global__ void __launch_bounds__(SCAN_THREADS) fuse_scan_kernel(const int* coun
 __global__ void __launch_bounds__(FUSE_THREADS, FUSE_BLOCKS) fuse_write_kernel(
     FuseArgs a, const unsigned* ballots, const long long* offsets, float* positions, float* normals, float* colors,
     long long capacity) {
-    __shared__ unsigned short list[FUSE_PIXELS];  // the CTA's emitted pixels in order
+    __shared__ unsigned short list[FUSE_STEPS * FUSE_THREADS];  // the CTA's emitted pixels in order
     __shared__ int listed;
     const long long base = offsets[blockIdx.x];
     if (threadIdx.x < 32) {  // one ballot word a lane
-        static_assert(FUSE_WORDS == 32, "one word a lane");
-        unsigned word = ballots[static_cast<size_t>(blockIdx.x) * FUSE_WORDS + threadIdx.x];
+        static_assert(FUSE_STEPS * STEP_WORDS == 32, "one word a lane");
+        const int words = a.steps * STEP_WORDS;
+        unsigned word =
+            threadIdx.x < words ? ballots[static_cast<size_t>(blockIdx.x) * words + threadIdx.x] : 0u;
         int at = __popc(word);
         for (int o = 1; o < 32; o <<= 1) {
             const int add = __shfl_up_sync(0xffffffffu, at, o);
@@ -299,7 +300,7 @@ __global__ void __launch_bounds__(FUSE_THREADS, FUSE_BLOCKS) fuse_write_kernel(
     __syncthreads();
     const int i = fuse_view_of(a, blockIdx.x);
     const int W = a.views[i].W;
-    const long long first = static_cast<long long>(blockIdx.x - a.view_block[i]) * FUSE_PIXELS;
+    const long long first = static_cast<long long>(blockIdx.x - a.view_block[i]) * a.steps * FUSE_THREADS;
     for (int k = threadIdx.x; k < listed; k += FUSE_THREADS) {
         const long long o = base + k;
         if (o >= capacity) break;

@@ -77,6 +77,7 @@ struct hp_ctx {
     hpx::DevBuf descs;   // ViewDesc array
     hpx::DevBuf lists;   // active-view lists and tile prefixes
     hpx::DevBuf staging; // host-memory results pass through here
+    hpx::DevBuf fuse;    // fusion descriptors, ballots and counts
     hpx::DevBuf seedbuf; // SfM seeds of one job and their W*H index map
     hpx::DevBuf upload;  // host images land here before conversion
     hpx::DevBuf filters; // FilterStage per filtered job of a solve

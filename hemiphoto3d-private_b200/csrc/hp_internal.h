@@ -10,10 +10,10 @@
 namespace hp {
 
 // Pixel tile one CTA covers: TILE_W x TILE_H pixels, 256 threads (the FP16
-// kernels also run TILE_W x 4 tiles with 128 threads).  In a
-// red-black half-pass each thread owns one pixel of the active color (a warp
-// covers one 64-pixel row segment); the full-map kernels give each thread the
-// two horizontally adjacent pixels of its pair.
+// kernels also run TILE_W x 4 tiles with 128 threads, and small per-pass
+// launches half a tile per CTA, split_tiles).  In a red-black half-pass each
+// thread owns one pixel of the active color (pass_pixel); in the full-map
+// kernels a warp takes 32 consecutive pixels at a time.
 constexpr int TILE_W = 64;
 constexpr int TILE_H = 8;
 constexpr int CTA_THREADS = 256;
@@ -223,11 +223,18 @@ struct FuseArgs {
     const int* neighbors;   // device
     const int* view_block;  // device, n_views + 1: first CTA of each view's pixels
     int n_views;
+    int steps;  // fuse_steps of the call
     int min_views;
     float min_conf, max_depth_rel, max_reproj_sq, min_normal_cos;
 };
 constexpr int FUSE_THREADS = 256;
-constexpr int FUSE_PIXELS = 1024;  // pixels per CTA of the fusion kernels, in four steps of FUSE_THREADS
+// Steps of FUSE_THREADS pixels a CTA of the fusion kernels takes.  Four give the
+// writing pass full warps where a third of the pixels emit; with one, small
+// inputs fill the GPU (FIGURES).  The line is two waves of four-step CTAs.
+constexpr int FUSE_STEPS = 4;
+inline int fuse_steps(long long pixels) {
+    return pixels >= 2ll * 148 * 6 * FUSE_STEPS * FUSE_THREADS ? FUSE_STEPS : 1;
+}
 
 }  // namespace hp
 
@@ -267,8 +274,8 @@ cudaError_t launch_filter_maps(const FilterMaps& a, float* depth, const float* n
                                cudaStream_t st);
 cudaError_t launch_to_f32(const void* src, int dtype, int W, int H, float* dst, int dst_pitch, __half* dst16,
                           int dst16_pitch, cudaStream_t st);
-// Fusion: per CTA the emitted pixels (FUSE_PIXELS / 32 ballot words) and their
-// number, the numbers' exclusive prefix (and the total), then the points
+// Fusion: per CTA the emitted pixels (ballot words, steps * FUSE_THREADS / 32) and
+// their number, the numbers' exclusive prefix (and the total), then the points
 // written at their offsets (index < capacity only).
 cudaError_t launch_fuse_count(const FuseArgs& a, int blocks, unsigned* ballots, int* block_counts, cudaStream_t st);
 cudaError_t launch_fuse_scan(const int* block_counts, int blocks, long long* block_offsets, long long* total,

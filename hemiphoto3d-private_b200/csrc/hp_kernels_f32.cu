@@ -208,10 +208,10 @@ __device__ __forceinline__ float cost_f32(const float* __restrict__ s_ref, int t
         // Not-a-numbers fail: `in` ignores them, the bound does not.
         inside = front && in > 0.0f && fmaf(fw1, Mz, Mx) <= 2e5f * zmin && fmaf(fh1, Mz, My) <= 2e5f * zmin;
     }
-#ifdef HP_COUNT_TAPS
-    atomicAdd(&g_taps32, static_cast<unsigned long long>(SIDE * SIDE));
-#endif
     if (!__any_sync(WARP, sampled)) return 2.0f;
+#ifdef HP_COUNT_TAPS
+    if (sampled) atomicAdd(&g_taps32, static_cast<unsigned long long>(SIDE * SIDE));
+#endif
     if (__all_sync(WARP, inside || !sampled)) {
         // Every tap of every sampled lane is valid: no tests, and the reference
         // sums are the window's own.  The same operations on the same values
