@@ -47,6 +47,11 @@ namespace {
 // with 2; one 320 x 240 view 1247, 1276 and 1262 us with 3, 4 and 2).
 template <int R, int ST>
 constexpr int pass_blocks() { return (2 * R) / ST + 1 <= 8 ? 4 : 3; }
+// Persistent launches: a small batch has fewer tiles at a stage than three CTAs
+// an SM, and the surplus CTAs wait on dependencies where others would run.  With
+// 2 and with pass_blocks(): 3 views up to 457 x 279, r 7, s 1, 5131 us and 7453;
+// 3 up to 320 x 240, r 3, s 2, 1176 and 1775; 3 up to 869 x 565 43.2 and 42.8 ms.
+constexpr int PERSISTENT_BLOCKS = 2;
 constexpr int COST_BLOCKS = 3;  // full-map cost, 1920 x 1080, r 5, s 1: 1486 us, 1574 with 2, 1506 with 4
 
 // Locate the view and tile of this CTA in a batch launch.
@@ -419,7 +424,7 @@ __global__ void __launch_bounds__(CTA_THREADS, pass_blocks<R, ST>()) propagate_k
 // bodies are the functions the per-stage kernels above run, so the results
 // are bit-identical to the per-stage launch sequence.
 template <int R, int ST>
-__global__ void __launch_bounds__(CTA_THREADS, pass_blocks<R, ST>()) persistent_kernel(Schedule s) {
+__global__ void __launch_bounds__(CTA_THREADS, PERSISTENT_BLOCKS) persistent_kernel(Schedule s) {
     __shared__ float s_ref[(TILE_W + 2 * R) * (TILE_H + 2 * R)];
     __shared__ Shared32<CTA_THREADS> sm;
     // The claimed tile lives in shared memory: warp 0 decodes it once and
