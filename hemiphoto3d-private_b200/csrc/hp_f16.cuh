@@ -628,6 +628,7 @@ template <int R, int ST, int TH, int D, int NT>
 struct Scorer16 {
     static constexpr int PX = 32 * TH, TW = TILE_W + 2 * R;
     static constexpr bool BLOCKS = !Win<R, ST>::IN_SMEM, BY_PLANE = false, WHOLE_WARPS = false;
+    static constexpr bool SMALL = Win<R, ST>::N <= 25;
     const ViewDesc* v;
     Shared<R, ST, TH, NT>& sm;
     int x0, y0;

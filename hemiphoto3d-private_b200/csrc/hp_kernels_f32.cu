@@ -374,6 +374,7 @@ struct Shared32 {
 template <int R, int ST, int PX>
 struct Scorer32 {
     static constexpr bool BLOCKS = true, BY_PLANE = true, WHOLE_WARPS = true;
+    static constexpr bool SMALL = ((2 * R) / ST + 1) * ((2 * R) / ST + 1) <= 25;
     const ViewDesc* v;
     const float* s_ref;
     Shared32<PX>& sm;

@@ -107,6 +107,7 @@ __device__ __forceinline__ int pass_thread(int lx, int ly) {
 //   mean(sum, k)                sum / k, monotone in sum
 //   BLOCKS                      pass_pixel's layout
 //   BY_PLANE                    neighbour items are listed by the plane they score, not by pixel
+//   SMALL                       windows of a few taps
 //   WHOLE_WARPS                 score needs all 32 lanes of a warp together
 template <int NT, int PX, class K>
 __device__ __forceinline__ void red_black_pass(const ViewDesc* v, int x0, int y0, const SolveConsts& sc,
@@ -185,8 +186,10 @@ __device__ __forceinline__ void red_black_pass(const ViewDesc* v, int x0, int y0
     // lane by lane: FP32, 2 x 1920 x 1080, 149.7 ms against 115.1).
     total = __shfl_sync(0xffffffffu, total, 0);
     const int kk = min(sc.top_k, S);
-    // With warps idle, two parts of few sources would take two turns where one takes one.
-    const int lead = roomy && S <= 3 ? S : S - kk + 1;
+    // With warps idle, two parts of few sources would take two turns where one takes one; with windows of a few taps and
+    // two sources the second part costs more than it saves (3 views up to 379 x 281, r 3, s 2, FP16-acc: 1864 us, whole
+    // 1692).
+    const int lead = (roomy && S <= 3) || (K::SMALL && S <= 2) ? S : S - kk + 1;
     float drange = __fmul_rn(__fsub_rn(v->dmax, v->dmin), 0.5f);
     float nrange = 1.0f;
     for (int i = 0; i < iteration; ++i) {
