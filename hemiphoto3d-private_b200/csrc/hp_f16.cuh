@@ -641,7 +641,7 @@ struct Scorer16 {
     __device__ __forceinline__ void set_plane(int k, int x, int y, float4 h, bool ok) {
         sm.plane[k] = ok ? plane_vector(v, x, y, h) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    __device__ __forceinline__ float score(int s, int k, int o, int lx, int ly) const {
+    __device__ __forceinline__ float score(int s, int k, int o, int lx, int ly, bool) const {
         const float2 os = sm.stat[o];
         const float4 m = sm.plane[k];
         if (m.w == 0.0f) return 2.0f;

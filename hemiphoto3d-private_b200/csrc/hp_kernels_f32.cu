@@ -213,11 +213,18 @@ __device__ __forceinline__ float cost_f32(const float* __restrict__ s_ref, int t
         // Not-a-numbers fail: `in` ignores them, the bound does not.
         inside = front && in > 0.0f && fmaf(fw1, Mz, Mx) <= 2e5f * zmin && fmaf(fh1, Mz, My) <= 2e5f * zmin;
     }
-    if (!__any_sync(WARP, sampled)) return 2.0f;
+    // The vote is the last step that needs the whole warp.  A lane without a
+    // window to sample (wholly outside, no plane, past the last item or the
+    // image) leaves here: while it ran along until the warp's last sampling lane
+    // was done, its fetches took the texture unit's time (1921 x 1081, 6 sources,
+    // cost of random planes: r 5 s 1 4166 -> 3991 us, r 7 s 2 2234 -> 2147; solve
+    // of 2 x 1920 x 1080, r 7, s 2: 93.9 -> 90.8 ms).
+    const bool all_inside = __all_sync(WARP, inside || !sampled);
+    if (!sampled) return 2.0f;
 #ifdef HP_COUNT_TAPS
-    if (sampled) atomicAdd(&g_taps32, static_cast<unsigned long long>(SIDE * SIDE));
+    atomicAdd(&g_taps32, static_cast<unsigned long long>(SIDE * SIDE));
 #endif
-    if (__all_sync(WARP, inside || !sampled)) {
+    if (all_inside) {
         // Every tap of every sampled lane is valid: no tests, and the reference
         // sums are the window's own.  The same operations on the same values
         // as below, so the same bits.
@@ -311,7 +318,7 @@ __device__ __forceinline__ float cost_f32(const float* __restrict__ s_ref, int t
             c = 1.0f - ncc;
         }
     }
-    return sampled ? c : 2.0f;
+    return c;
 }
 
 __global__ void __launch_bounds__(256) init_kernel(BatchList bl) {
@@ -338,15 +345,17 @@ __device__ __forceinline__ void tile_cost(const ViewDesc* v, int x0, int y0, con
     const int ly = warp / WARPS_A_ROW, y = y0 + ly;
     if (y >= v->H) return;
     for (int j = 0; j < 2 / WARPS_A_ROW; ++j) {
-        // Whole warps score; lanes past the image repeat its last column.
+        // Whole warps vote; lanes past the image name its last column and neither sample nor store.
         const int left = 32 * (j + warp % WARPS_A_ROW), lx = min(left + lane, v->W - 1 - x0), x = x0 + lx;
         if (lx < left) break;
         const size_t idx = static_cast<size_t>(y) * v->W + x;
-        const PlaneF32 p = plane_f32(v, x, y, v->hyp[idx]);
+        PlaneF32 p = plane_f32(v, x, y, v->hyp[idx]);
+        const bool live = left + lane == lx;
+        p.ok = p.ok && live;
         const float2 sums = window_sums<R, ST>(s_ref, tw, lx, ly);
         Lowest low;
         for (int s = 0; s < v->S; ++s) low.insert(cost_f32<R, ST>(s_ref, tw, lx, ly, x, y, p, sums, v, s));
-        v->cost[idx] = mean_f32(low.sum(min(sc.top_k, v->S)), min(sc.top_k, v->S));
+        if (live) v->cost[idx] = mean_f32(low.sum(min(sc.top_k, v->S)), min(sc.top_k, v->S));
     }
 }
 
@@ -388,10 +397,10 @@ struct Scorer32 {
         sm.plane[k] = make_float4(p.nK0, p.nK1, p.nK2, p.inv_n_dot_P);
         sm.ok[k] = ok && p.ok;
     }
-    __device__ __forceinline__ float score(int s, int k, int o, int lx, int ly) const {
+    __device__ __forceinline__ float score(int s, int k, int o, int lx, int ly, bool live) const {
         const float4 q = sm.plane[k];
-        return cost_f32<R, ST>(s_ref, TILE_W + 2 * R, lx, ly, x0 + lx, y0 + ly, PlaneF32{q.x, q.y, q.z, q.w, sm.ok[k] != 0},
-                               sm.sums[o], v, s);
+        return cost_f32<R, ST>(s_ref, TILE_W + 2 * R, lx, ly, x0 + lx, y0 + ly,
+                               PlaneF32{q.x, q.y, q.z, q.w, live && sm.ok[k] != 0}, sm.sums[o], v, s);
     }
     __device__ __forceinline__ float mean(float sum, int k) const { return mean_f32(sum, k); }
 };

@@ -103,12 +103,13 @@ __device__ __forceinline__ int pass_thread(int lx, int ly) {
 //   begin(lx, ly)               prepares the window of the thread's own pixel (active pixels only)
 //   publish()                   makes it readable by the other threads (after the next barrier)
 //   set_plane(k, x, y, h, ok)   thread k: plane h of item k at pixel (x, y), ok false: no plane
-//   score(source, k, o, lx, ly) cost of item k, whose pixel is thread o's, at tile position (lx, ly)
+//   score(source, k, o, lx, ly, live)  cost of item k, whose pixel is thread o's, at tile position (lx, ly); lanes
+//                               that are not live take part for their warp's sake
 //   mean(sum, k)                sum / k, monotone in sum
 //   BLOCKS                      pass_pixel's layout
 //   BY_PLANE                    neighbour items are listed by the plane they score, not by pixel
 //   SMALL                       windows of a few taps
-//   WHOLE_WARPS                 score needs all 32 lanes of a warp together
+//   WHOLE_WARPS                 score starts with a vote of all 32 lanes of a warp
 template <int NT, int PX, class K>
 __device__ __forceinline__ void red_black_pass(const ViewDesc* v, int x0, int y0, const SolveConsts& sc,
                                                int iteration, int color, K& scorer, float* unit,
@@ -252,13 +253,15 @@ __device__ __forceinline__ void red_black_pass(const ViewDesc* v, int x0, int y0
                     const int turn = (q - first) * ((units + 31) >> 5);
 #pragma unroll 1
                     for (int u0 = ((warp - turn) & (NT / 32 - 1)) * 32; u0 < units; u0 += NT) {
-                        // A scorer that votes wants whole warps: the last lanes repeat the last item.
+                        // A scorer that votes wants whole warps: lanes past the last item name it too and are not live.
                         const int u = K::WHOLE_WARPS ? min(u0 + lane, units - 1) : u0 + lane;
-                        if (!K::WHOLE_WARPS && u >= units) continue;
+                        const bool live = u0 + lane < units;
+                        if (!K::WHOLE_WARPS && !live) continue;
                         const int k = first > 0 ? sm.items[u] : u;
                         const int o = round == 0 ? sm.items[c0 + k] >> 2 : k;
                         const int2 at = pass_pixel<K::BLOCKS>(o, y0, color);
-                        unit[q * NT + k] = scorer.score(source, k, o, at.x, at.y);
+                        const float cost = scorer.score(source, k, o, at.x, at.y, live);
+                        if (live) unit[q * NT + k] = cost;
                     }
                 }
                 __syncthreads();  // the part's source costs are complete
