@@ -262,6 +262,7 @@ struct Prepared {
     std::vector<int> list_offsets;    // per iteration: offset into lists buffer
     std::vector<int> list_counts;     // per iteration: number of active views
     std::vector<int> list_tiles;      // per iteration: total tiles
+    std::vector<int> list_sources;    // per iteration: the most sources of a view
     int* lists = nullptr;
     int max_iter = 0;
     std::vector<int> filter_order;    // jobs with a filter stage, in the order they run
@@ -338,6 +339,9 @@ hp_status prepare(hp_ctx* ctx, const hp_job* jobs, int n, const hp_params* param
         }
         ints.push_back(acc);
         P->list_tiles.push_back(acc);
+        int sources = 0;
+        for (int k : act) sources = std::max(sources, P->host[k].S);
+        P->list_sources.push_back(sources);
     }
     HP_CUDA(ctx->lists.ensure(ints.size() * sizeof(int)));
     P->lists = static_cast<int*>(ctx->lists.p);
@@ -356,6 +360,7 @@ hp::BatchList batch_of(const Prepared& P, int list) {
     bl.active = P.lists + P.list_offsets[list];
     bl.tile_prefix = bl.active + bl.n_active;
     bl.total_tiles = P.list_tiles[list];
+    bl.max_sources = P.list_sources[list];
     return bl;
 }
 

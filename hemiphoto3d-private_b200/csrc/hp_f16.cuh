@@ -108,14 +108,15 @@ struct RefStats {
 // Shared memory of a CTA (dynamic: the widest windows pass the 48 KB static
 // limit).  Windows kept in s_win need the reference tile only while they are
 // built, so the half-pass's source costs then take its place.
-template <int R, int ST, int TH, int THREADS = 32 * TH>
+template <int R, int ST, int TH, int THREADS = 32 * TH, PassForm F = PassForm::UNITS>
 struct alignas(16) Shared {
+    static constexpr bool WHOLE = F == PassForm::WHOLE;
     static constexpr int NT = THREADS, PX = 32 * TH;  // threads, active pixels of a half-pass
     static constexpr int REF = (TILE_W + 2 * R) * (TH + 2 * R);
-    static constexpr int UNITS = HP_MAX_SOURCES * NT;
+    static constexpr int UNITS = WHOLE ? 1 : HP_MAX_SOURCES * NT;
     static constexpr bool OVERLAY = Win<R, ST>::IN_SMEM;
     __half2 win[OVERLAY ? Win<R, ST>::SIDE * Win<R, ST>::VEC * PX : 4];  // see load_window
-    float4 plane[NT];               // half-pass: plane_vector of the chunk's items
+    float4 plane[WHOLE ? 1 : NT];   // half-pass: plane_vector of the chunk's items
     float ref[OVERLAY ? (REF > UNITS ? REF : UNITS) : REF];
     float unit_own[OVERLAY ? 1 : UNITS];
     float2 stat[PX];                // half-pass: (mean, ssd) of each pixel's window
@@ -578,14 +579,13 @@ __device__ __forceinline__ float unit_cost(const ViewDesc* __restrict__ v, int s
 }
 
 extern __shared__ __align__(16) unsigned char dynamic_smem[];
-template <int R, int ST, int TH, int NT = 32 * TH>
-__device__ __forceinline__ Shared<R, ST, TH, NT>& shared_of() {
-    return *reinterpret_cast<Shared<R, ST, TH, NT>*>(dynamic_smem);
+template <class S>
+__device__ __forceinline__ S& shared_of() {
+    return *reinterpret_cast<S*>(dynamic_smem);
 }
 
-template <int R, int ST, int TH, int D>
-__device__ __forceinline__ void tile_cost16(const ViewDesc* v, int tile_x, int tile_y, const SolveConsts& sc,
-                                            Shared<R, ST, TH>& sm) {
+template <int R, int ST, int TH, int D, class S>
+__device__ __forceinline__ void tile_cost16(const ViewDesc* v, int tile_x, int tile_y, const SolveConsts& sc, S& sm) {
     constexpr int NT = Tile<TH>::NT;
     float* s_ref = sm.ref;
     __half2* s_win = sm.win;
@@ -619,18 +619,19 @@ template <int R, int ST, int TH, int D>
 __global__ void __launch_bounds__(Tile<TH>::NT, Tile<TH>::MIN_BLOCKS) cost16_kernel(BatchList bl, SolveConsts sc) {
     int tile_x, tile_y;
     const ViewDesc* v = locate_tile16(bl, blockIdx.x, &tile_x, &tile_y);
-    tile_cost16<R, ST, TH, D>(v, tile_x, tile_y, sc, shared_of<R, ST, TH>());
+    tile_cost16<R, ST, TH, D>(v, tile_x, tile_y, sc, shared_of<Shared<R, ST, TH>>());
 }
 
 // Scorer of the half-pass (red_black_pass): a unit reads its pixel's window
 // statistics and s_win column, and its item's plane vector, from shared memory.
-template <int R, int ST, int TH, int D, int NT>
+template <int R, int ST, int TH, int D, int NT, PassForm F>
 struct Scorer16 {
     static constexpr int PX = 32 * TH, TW = TILE_W + 2 * R;
     static constexpr bool BLOCKS = !Win<R, ST>::IN_SMEM, BY_PLANE = false, WHOLE_WARPS = false;
-    static constexpr bool SMALL = Win<R, ST>::N <= 25;
+    static constexpr PassForm FORM = F;
+    using Plane = float4;
     const ViewDesc* v;
-    Shared<R, ST, TH, NT>& sm;
+    Shared<R, ST, TH, NT, F>& sm;
     int x0, y0;
     unsigned soft_mask;
     RefStats st{0.f, 0.f};
@@ -638,46 +639,51 @@ struct Scorer16 {
     __device__ __forceinline__ void publish() {
         if (NT == PX || threadIdx.x < PX) sm.stat[threadIdx.x] = make_float2(st.mean, st.ssd);
     }
-    __device__ __forceinline__ void set_plane(int k, int x, int y, float4 h, bool ok) {
-        sm.plane[k] = ok ? plane_vector(v, x, y, h) : make_float4(0.f, 0.f, 0.f, 0.f);
+    __device__ __forceinline__ float4 plane(int x, int y, float4 h, bool ok) const {
+        return ok ? plane_vector(v, x, y, h) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    __device__ __forceinline__ float score(int s, int k, int o, int lx, int ly, bool) const {
+    __device__ __forceinline__ bool has(float4 m) const { return m.w != 0.0f; }
+    __device__ __forceinline__ void store(int k, float4 m) { sm.plane[k] = m; }
+    __device__ __forceinline__ float4 load(int k) const { return sm.plane[k]; }
+    __device__ __forceinline__ float score(int s, float4 m, int o, int lx, int ly, bool) const {
         const float2 os = sm.stat[o];
-        const float4 m = sm.plane[k];
-        if (m.w == 0.0f) return 2.0f;
         return unit_cost<R, ST, PX, D>(v, s, m.x, m.y, m.z, RefStats{os.x, os.y}, sm.win + o * Win<R, ST>::VEC,
                                        sm.ref, TW, lx, ly, x0 + lx, y0 + ly, soft_mask);
     }
     __device__ __forceinline__ float mean(float sum, int k) const { return __fdiv_rn(sum, static_cast<float>(k)); }
 };
 
-template <int R, int ST, int TH, int D, int NT>
+template <int R, int ST, int TH, int D, int NT, PassForm F>
 __device__ __forceinline__ void tile_propagate16(const ViewDesc* v, int x0, int y0, const SolveConsts& sc,
-                                                 int iteration, int color, Shared<R, ST, TH, NT>& sm,
-                                                 bool roomy = false) {
+                                                 int iteration, int color, Shared<R, ST, TH, NT, F>& sm) {
     load_ref_tile16<NT>(sm.ref, TILE_W + 2 * R, TH + 2 * R, v, x0, y0, R);
     __syncthreads();
-    Scorer16<R, ST, TH, D, NT> scorer{v, sm, x0, y0, sc.soft_mask};
-    red_black_pass<NT, 32 * TH>(v, x0, y0, sc, iteration, color, scorer, sm.units(), sm.pass, roomy);
+    Scorer16<R, ST, TH, D, NT, F> scorer{v, sm, x0, y0, sc.soft_mask};
+    red_black_pass<NT, 32 * TH>(v, x0, y0, sc, iteration, color, scorer, sm.units(), sm.pass);
 }
 
-// SPLIT: two CTAs of half the tile's rows and all its threads to a tile (split_tiles).
-template <int R, int ST, int TH, int D, bool SPLIT>
+// Rows and shared memory of a half-pass CTA: half tiles keep all of the tile's threads.
+template <int R, int ST, int TH, PassForm F>
+struct PassShape {
+    static constexpr bool HALVES = F == PassForm::ROOMY || F == PassForm::SPLIT;
+    static constexpr int ROWS = HALVES ? TH / 2 : TH;
+    using Smem = Shared<R, ST, ROWS, Tile<TH>::NT, F>;
+};
+template <int R, int ST, int TH, int D, PassForm F>
 __global__ void __launch_bounds__(Tile<TH>::NT, Tile<TH>::MIN_BLOCKS) propagate16_kernel(BatchList bl, SolveConsts sc,
-                                                                                       int iteration, int color,
-                                                                                       bool roomy) {
-    constexpr int ROWS = SPLIT ? TH / 2 : TH, NT = Tile<TH>::NT;
+                                                                                       int iteration, int color) {
+    using P = PassShape<R, ST, TH, F>;
     int tile_x, tile_y;
-    const ViewDesc* v = locate_tile16(bl, SPLIT ? blockIdx.x >> 1 : blockIdx.x, &tile_x, &tile_y);
-    tile_propagate16<R, ST, ROWS, D, NT>(v, tile_x * TILE_W, tile_y * TH + (SPLIT ? (blockIdx.x & 1) * ROWS : 0), sc,
-                                         iteration, color, shared_of<R, ST, ROWS, NT>(), roomy);
+    const ViewDesc* v = locate_tile16(bl, P::HALVES ? blockIdx.x >> 1 : blockIdx.x, &tile_x, &tile_y);
+    const int y0 = tile_y * TH + (P::HALVES ? (blockIdx.x & 1) * P::ROWS : 0);
+    tile_propagate16<R, ST, P::ROWS, D>(v, tile_x * TILE_W, y0, sc, iteration, color, shared_of<typename P::Smem>());
 }
 
 // Persistent form (see Schedule and the FP32 persistent kernel): the stage
 // bodies are those of the per-stage kernels, so the results are bit-identical.
-template <int R, int ST, int TH, int D>
+template <int R, int ST, int TH, int D, PassForm F>
 __global__ void __launch_bounds__(Tile<TH>::NT, Tile<TH>::MIN_BLOCKS) persistent16_kernel(Schedule s) {
-    Shared<R, ST, TH>& sm = shared_of<R, ST, TH>();
+    auto& sm = shared_of<Shared<R, ST, TH, Tile<TH>::NT, F>>();
     // The claimed tile lives in shared memory: warp 0 decodes it once and
     // thread 0 publishes it after the stage, so no thread carries it through the body.
     __shared__ SchedTile s_tile;
@@ -714,7 +720,7 @@ __global__ void __launch_bounds__(Tile<TH>::NT, Tile<TH>::MIN_BLOCKS) persistent
             tile_cost16<R, ST, TH, D>(v, tx, ty, s.sc, sm);
         } else if (stage <= 2 * v->iterations) {
             const int k = stage - 1;
-            tile_propagate16<R, ST, TH, D, Tile<TH>::NT>(v, tx * TILE_W, ty * TH, s.sc, k >> 1, k & 1, sm);
+            tile_propagate16<R, ST, TH, D>(v, tx * TILE_W, ty * TH, s.sc, k >> 1, k & 1, sm);
         } else if (is_filter_stage(v, stage)) {
             tile_filter(s.views, v, tx, ty, true);  // geometric check, then the maps
         } else {
@@ -731,43 +737,59 @@ __global__ void __launch_bounds__(Tile<TH>::NT, Tile<TH>::MIN_BLOCKS) persistent
 // 2: persistent (occ non-null: occupancy query only).
 template <int TH>
 struct Dispatch {
+    // Launches f with shared memory of type S, opting in to more than 48 KB on the current device (a property of
+    // the function there; setting it again is harmless).
+    template <class S, class... A>
+    static cudaError_t launch(void (*f)(A...), int grid, cudaStream_t st, A... args) {
+        constexpr int smem = static_cast<int>(sizeof(S));
+        const cudaError_t e = cudaFuncSetAttribute(reinterpret_cast<const void*>(f),
+                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e != cudaSuccess) return e;
+        f<<<grid, Tile<TH>::NT, smem, st>>>(args...);
+        return cudaGetLastError();
+    }
+    template <int R, int ST, int D, PassForm F>
+    static cudaError_t persistent(const Schedule& s, int grid, cudaStream_t st, int* occ) {
+        using S = Shared<R, ST, TH, Tile<TH>::NT, F>;
+        if (!occ) return launch<S>(persistent16_kernel<R, ST, TH, D, F>, grid, st, s);
+        constexpr int smem = static_cast<int>(sizeof(S));
+        const cudaError_t e =
+            cudaFuncSetAttribute(reinterpret_cast<const void*>(persistent16_kernel<R, ST, TH, D, F>),
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e != cudaSuccess) return e;
+        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, persistent16_kernel<R, ST, TH, D, F>, Tile<TH>::NT,
+                                                             smem);
+    }
+    template <int R, int ST, int D, PassForm F>
+    static cudaError_t pass(const BatchList& bl, const SolveConsts& sc, int iteration, int color, cudaStream_t st) {
+        using P = PassShape<R, ST, TH, F>;
+        return launch<typename P::Smem>(propagate16_kernel<R, ST, TH, D, F>, bl.total_tiles * (P::HALVES ? 2 : 1), st,
+                                        bl, sc, iteration, color);
+    }
+    // The forms other than UNITS keep four loads in flight: the staging depth changes no bit.
     template <int R, int ST, int D>
     static cudaError_t run(int mode, const BatchList* bl, const SolveConsts& sc, int iteration, int color,
                            const Schedule* s, int grid, cudaStream_t st, int* occ) {
-        constexpr int NT = Tile<TH>::NT;
-        constexpr int smem = static_cast<int>(sizeof(Shared<R, ST, TH>));
-        // Opt in to more than 48 KB on the current device (a property of the function there; setting it again
-        // is harmless).
-        auto allow = [](const void* f) {
-            return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        };
-        cudaError_t e;
+        constexpr int N = Win<R, ST>::N;
         if (mode == 2) {
-            if ((e = allow(reinterpret_cast<const void*>(persistent16_kernel<R, ST, TH, D>))) != cudaSuccess) return e;
-            if (occ)
-                return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, persistent16_kernel<R, ST, TH, D>, NT, smem);
-            persistent16_kernel<R, ST, TH, D><<<grid, NT, smem, st>>>(*s);
-        } else if (mode == 0) {
-            if ((e = allow(reinterpret_cast<const void*>(cost16_kernel<R, ST, TH, D>))) != cudaSuccess) return e;
-            cost16_kernel<R, ST, TH, D><<<bl->total_tiles, NT, smem, st>>>(*bl, sc);
-        } else {
-            if constexpr (TH == 8) {
-                const int sms = device_sms();
-                if (split_tiles(bl->total_tiles, sms)) {  // 4 loads in flight: the staging depth changes no bit
-                    constexpr int half = static_cast<int>(sizeof(Shared<R, ST, TH / 2, NT>));
-                    if ((e = cudaFuncSetAttribute(propagate16_kernel<R, ST, TH, 4, true>,
-                                                  cudaFuncAttributeMaxDynamicSharedMemorySize, half)) != cudaSuccess)
-                        return e;
-                    propagate16_kernel<R, ST, TH, 4, true><<<2 * bl->total_tiles, NT, half, st>>>(
-                        *bl, sc, iteration, color, 2 * bl->total_tiles <= 3 * sms);
-                    return cudaGetLastError();
-                }
-            }
-            if ((e = allow(reinterpret_cast<const void*>(propagate16_kernel<R, ST, TH, D, false>))) != cudaSuccess)
-                return e;
-            propagate16_kernel<R, ST, TH, D, false><<<bl->total_tiles, NT, smem, st>>>(*bl, sc, iteration, color, false);
+            if constexpr (N <= PASS_RULE_F16.whole_persistent)
+                if (persistent_whole(PASS_RULE_F16, N, s->max_sources, s->tiles, device_sms()))
+                    return persistent<R, ST, 4, PassForm::WHOLE>(*s, grid, st, occ);
+            return persistent<R, ST, D, PassForm::UNITS>(*s, grid, st, occ);
         }
-        return cudaGetLastError();
+        if (mode == 0)
+            return launch<Shared<R, ST, TH>>(cost16_kernel<R, ST, TH, D>, bl->total_tiles, st, *bl, sc);
+        const PassForm form = pass_form(sc.memo ? PASS_RULE_F16 : PASS_RULE_F16_SINGLE, N, bl->max_sources,
+                                        bl->total_tiles, device_sms());
+        if constexpr (TH == 8) {
+            if (form == PassForm::ROOMY) return pass<R, ST, 4, PassForm::ROOMY>(*bl, sc, iteration, color, st);
+            if (form == PassForm::SPLIT) return pass<R, ST, 4, PassForm::SPLIT>(*bl, sc, iteration, color, st);
+        }
+        // Units earn their keep by the trial bound; a half-pass on caller maps goes without it (1921 x 1081, whole call,
+        // units -> whole: r 7 s 2, 6 sources 3329 -> 3201 us, 1 source 692 -> 641; r 1 s 1, 6 sources 941 -> 783).
+        if (form == PassForm::WHOLE || !sc.memo)
+            return pass<R, ST, 4, PassForm::WHOLE>(*bl, sc, iteration, color, st);
+        return pass<R, ST, D, PassForm::UNITS>(*bl, sc, iteration, color, st);
     }
     template <int R, int ST>
     static cudaError_t depth(int mode, int staging, const BatchList* bl, const SolveConsts& sc, int iteration,

@@ -5,13 +5,15 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
+
 #include "../../include/hpmvs.h"
 
 namespace hp {
 
 // Pixel tile one CTA covers: TILE_W x TILE_H pixels, 256 threads (the FP16
 // kernels also run TILE_W x 4 tiles with 128 threads, and small per-pass
-// launches half a tile per CTA, split_tiles).  In a red-black half-pass each
+// launches half a tile per CTA, PassForm).  In a red-black half-pass each
 // thread owns one pixel of the active color (pass_pixel); in the full-map
 // kernels a warp takes 32 consecutive pixels at a time.
 constexpr int TILE_W = 64;
@@ -85,22 +87,60 @@ struct SolveConsts {
     int memo;            // half-passes keep and use the settled bit of stored costs (whole solves: 1)
 };
 
-// Small per-pass launches can run two CTAs on each 64 x 8 tile, 64 x 4 pixels
-// with the same 256 threads.  That pays
-//  - up to one tile an SM: a GPU that is not full gets twice the warps, and each
-//    takes half as many turns of (item, source) units;
-//  - beyond, when half tiles spread better: the busiest SM's share is
-//    ceil(2 t / SMs) halves instead of 2 ceil(t / SMs), less when the part of
-//    t / SMs past its whole number lies in (0, 1/2].  Past 8 tiles an SM there is
-//    little left to gain.
-// Measured, whole tiles -> halves (148 SMs): FP16-acc r 7 s 2, 4 sources, 8
-// iterations, 320 x 240 (150 tiles) 1914 -> 1540 us, 480 x 360 (360) 2708 ->
-// 2385, 560 x 420 (477) 3119 -> 2915, but 400 x 300 (266) 1965 -> 2006 and 720 x
-// 540 (816) 4210 -> 4254; FP32 r 5 s 1, 320 x 240, 2 sources, 4 iterations 1154
-// -> 975 us, 480 x 360, 6 sources 7353 -> 6703, 400 x 300 3779 -> 4007.
-inline bool split_tiles(int tiles, int sms) {
-    const int past = tiles % sms;
-    return tiles <= sms || (tiles <= 8 * sms && past > 0 && 2 * past <= sms);
+// What a launch of half-passes runs (red_black_pass), by what fills its SMs.
+//  UNITS  one CTA a tile, scoring in (item, source) units.
+//  ROOMY  two CTAs a tile, 64 x 4 pixels with the same 256 threads, up to 3 / 2 tiles
+//         an SM: a GPU that is not full gets twice the warps, and each takes half as
+//         many turns of units.
+//  SPLIT  the same beyond, where half tiles spread better: the busiest SM's share is
+//         ceil(2 t / SMs) halves instead of 2 ceil(t / SMs), less when the part of
+//         t / SMs past its whole number lies in (0, 1/2].  Half tiles cost more halo
+//         and leave half the threads of a part of few units idle, so the more tiles
+//         an SM has, the more window samples a pixel needs for them to pay.
+//  WHOLE  one CTA a tile, a thread scoring all sources of its item: no shared planes,
+//         no stored unit costs and no barriers between trials, but no trial bound.
+//         It pays while a pixel has few window samples.
+enum class PassForm { UNITS, ROOMY, SPLIT, WHOLE };
+constexpr int window_taps(int radius, int stride) { return ((2 * radius) / stride + 1) * ((2 * radius) / stride + 1); }
+// The lines between them, in window samples of a pixel's plane (taps x sources), and
+// what both sides measured on 148 SMs, us a solve of 6 or 8 iterations:
+//  whole: FP16-acc 961 x 541, units -> whole: r 1 s 1, 1 source 993 -> 841, 6
+//   sources 2398 -> 2285; r 3 s 2, 3 sources 1923 -> 1845; 1921 x 1081, r 3 s 1, 3
+//   sources (147) 11100 units, 12345 whole.  FP32 573 x 303: r 1 s 1, 1 source
+//   377 -> 342; r 3 s 2, 2 sources (32) 575 units, 563 whole.
+//  split, S >= 3 / S < 3: tiles an SM up to which half tiles win.  FP16-acc, units ->
+//   halves: r 3 s 1, 3 sources (147) 2.3 tiles an SM 1232 -> 1199, 5.1 2036 -> 2127;
+//   r 7 s 2, 8 sources (512) 4.5 5206 -> 4896, 7.4 7732 -> 7660; 2 sources (128) 2.1
+//   1235 -> 1195, 2.3 1169 -> 1234.  FP32: r 5 s 2, 3 sources (108) 4.5 1925 -> 1891,
+//   6.1 2385 -> 2408; r 7 s 2, 2 sources (128) 2.1 1291 -> 1322; r 5 s 1, 2 sources
+//   (242) 2.3 2610 -> 2426, 3.1 2880 -> 2930.
+//  A single half-pass on caller maps has no trial bound, so units gain by halves alone:
+//   FP16-acc 641 x 479 (4.1 tiles an SM), r 7 s 2, 3 sources 323 whole, 306 halves.
+struct PassRule {
+    int whole, whole_persistent;  // WHOLE up to so many samples, in per-pass and in persistent launches
+    int many, few;                // SPLIT up to samples / many (three or more sources) or samples / few tiles an SM,
+    float many_max, few_max;      // and up to these
+};
+constexpr PassRule PASS_RULE_F32{27, 64, 24, 100, 8.0f, 8.0f};
+constexpr PassRule PASS_RULE_F16{100, 100, 50, 100, 8.0f, 2.25f};
+constexpr PassRule PASS_RULE_F16_SINGLE{100, 100, 25, 30, 5.0f, 5.0f};
+inline bool roomy_tiles(int tiles, int sms) { return 2 * tiles <= 3 * sms; }
+inline bool halves_spread(int tiles, int sms) { return tiles % sms > 0 && 2 * (tiles % sms) <= sms; }
+inline bool split_cost(int tiles, int sms) { return tiles <= sms || (tiles <= 8 * sms && halves_spread(tiles, sms)); }
+// A persistent launch has no half tiles, so only the bound speaks against whole items: where SMs idle it saves turns
+// (one 160 x 120 view, FP16-acc, r 2 s 1, 4 sources 1066 us in units, 1277 whole; r 2 s 2, 1 source 445 and 402), else
+// work (3 views of 379 x 281, FP32, r 2 s 2, 2 sources 994 and 902).
+inline bool persistent_whole(const PassRule& r, int taps, int max_sources, int tiles, int sms) {
+    const int samples = taps * max_sources;
+    return samples <= (roomy_tiles(tiles, sms) && max_sources > 1 ? 36 : r.whole_persistent);
+}
+inline PassForm pass_form(const PassRule& r, int taps, int max_sources, int tiles, int sms) {
+    const int samples = taps * max_sources;
+    if (roomy_tiles(tiles, sms)) return PassForm::ROOMY;
+    if (samples <= r.whole) return PassForm::WHOLE;
+    const float most = max_sources >= 3 ? std::min(r.many_max, static_cast<float>(samples) / r.many)
+                                        : std::min(r.few_max, static_cast<float>(samples) / r.few);
+    return halves_spread(tiles, sms) && tiles <= most * sms ? PassForm::SPLIT : PassForm::UNITS;
 }
 inline int device_sms() {
     int dev = 0, sms = 148;
@@ -116,6 +156,7 @@ struct BatchList {
     const int* tile_prefix;     // n_active + 1 entries
     int n_active;
     int total_tiles;
+    int max_sources;            // of the active views
 };
 
 // Persistent launch.  A view's work is a sequence of stages, each covering
@@ -154,6 +195,7 @@ struct Schedule {
     int* status;                  // [0] SCHED_* code, [1] abort flag, [2] ticket whose wait ran out
     int* abort;                   // abort flag (null: status + 1; the launchers fill it in)
     unsigned long long wait_limit_ns;
+    int tiles, max_sources;       // tiles of the views together, the most sources of one
     int stall_view, stall_tile;   // this tile never reports completion (bounded-wait test); -1 = none
     SolveConsts sc;
     // Filter stages (null when the schedule has none): tickets below
@@ -249,9 +291,9 @@ cudaError_t launch_propagate_f32(const BatchList& bl, const SolveConsts& sc, int
 cudaError_t launch_cost_f16(const BatchList& bl, const SolveConsts& sc, cudaStream_t st);
 cudaError_t launch_persistent_f32(const Schedule& s, int grid, cudaStream_t st);
 cudaError_t launch_persistent_f16(const Schedule& s, int grid, cudaStream_t st);
-// Resident CTAs per SM of the persistent kernel for (radius, stride).
-cudaError_t persistent_occupancy_f32(int radius, int stride, int* blocks_per_sm);
-cudaError_t persistent_occupancy_f16(const SolveConsts& sc, int* blocks_per_sm);
+// Resident CTAs per SM of the persistent kernel that views of so many tiles and sources take.
+cudaError_t persistent_occupancy_f32(const SolveConsts& sc, int tiles, int max_sources, int* blocks_per_sm);
+cudaError_t persistent_occupancy_f16(const SolveConsts& sc, int tiles, int max_sources, int* blocks_per_sm);
 cudaError_t launch_propagate_f16(const BatchList& bl, const SolveConsts& sc, int iteration, int color,
                                  cudaStream_t st);
 // FP16 plane -> block-tiled software-sampler quad plane (see hpx::QuadPlane).

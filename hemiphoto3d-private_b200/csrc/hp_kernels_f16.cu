@@ -49,8 +49,11 @@ cudaError_t launch_persistent_f16(const Schedule& s, int grid, cudaStream_t st) 
     return dispatch(2, k.sc.tile_h, k.sc, nullptr, 0, 0, &k, grid, st, nullptr);
 }
 
-cudaError_t persistent_occupancy_f16(const SolveConsts& sc, int* blocks_per_sm) {
-    return dispatch(2, sc.tile_h, sc, nullptr, 0, 0, nullptr, 0, nullptr, blocks_per_sm);
+cudaError_t persistent_occupancy_f16(const SolveConsts& sc, int tiles, int max_sources, int* blocks_per_sm) {
+    Schedule s{};
+    s.tiles = tiles;
+    s.max_sources = max_sources;
+    return dispatch(2, sc.tile_h, sc, nullptr, 0, 0, &s, 0, nullptr, blocks_per_sm);
 }
 
 }  // namespace hp

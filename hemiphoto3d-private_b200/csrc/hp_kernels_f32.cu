@@ -45,8 +45,14 @@ namespace {
 // (2 x 1920 x 1080, r 7, s 2: 97.9 ms, against 99.9 with 3 CTAs and 108.8 with
 // 2); longer rows want 80 (5 x 640 x 480, r 5, s 1: 45.9 ms with 3 or 4, 48.3
 // with 2; one 320 x 240 view 1247, 1276 and 1262 us with 3, 4 and 2).
-template <int R, int ST>
-constexpr int pass_blocks() { return (2 * R) / ST + 1 <= 8 ? 4 : 3; }
+// Launches with at most three CTAs for an SM have nothing to gain from a fourth
+// (253 x 175, r 3 s 1, 3 sources, 6 iterations 664 -> 639 us; r 1 s 1, 1 source 260
+// -> 254), and whole items (PassForm::WHOLE) spill at 64 registers (573 x 303, r 1
+// s 1, 1 source 353 -> 342 us).
+template <int R, int ST, PassForm F>
+constexpr int pass_blocks() {
+    return F == PassForm::ROOMY || F == PassForm::WHOLE || (2 * R) / ST + 1 > 8 ? 3 : 4;
+}
 // Persistent launches: a small batch has fewer tiles at a stage than three CTAs
 // an SM, and the surplus CTAs wait on dependencies where others would run.  With
 // 2 and with pass_blocks(): 3 views up to 457 x 279, r 7, s 1, 5131 us and 7453;
@@ -359,7 +365,7 @@ __device__ __forceinline__ void tile_cost(const ViewDesc* v, int x0, int y0, con
     }
 }
 
-// SPLIT: two CTAs of 64 x 4 pixels to a tile (split_tiles).
+// SPLIT: two CTAs of 64 x 4 pixels to a tile (split_cost).
 template <int R, int ST, bool SPLIT>
 __global__ void __launch_bounds__(CTA_THREADS, COST_BLOCKS) cost_kernel(BatchList bl, SolveConsts sc) {
     constexpr int TH = SPLIT ? TILE_H / 2 : TILE_H;
@@ -370,73 +376,83 @@ __global__ void __launch_bounds__(CTA_THREADS, COST_BLOCKS) cost_kernel(BatchLis
 }
 
 // Shared memory of a half-pass beyond the reference tile.
-template <int PX>
+template <int PX, PassForm F>
 struct Shared32 {
-    float4 plane[CTA_THREADS];  // nK and 1 / (n.P) of the chunk's items
-    float unit[HP_MAX_SOURCES * CTA_THREADS];
-    unsigned char ok[CTA_THREADS];
+    static constexpr bool WHOLE = F == PassForm::WHOLE;
+    float4 plane[WHOLE ? 1 : CTA_THREADS];  // nK and 1 / (n.P) of the chunk's items
+    float unit[WHOLE ? 1 : HP_MAX_SOURCES * CTA_THREADS];
+    unsigned char ok[WHOLE ? 1 : CTA_THREADS];
     float2 sums[PX];            // window_sums of each pixel
     PassShared<CTA_THREADS, PX> pass;
 };
 
 // Scorer of the half-pass (red_black_pass).
-template <int R, int ST, int PX>
+template <int R, int ST, int PX, PassForm F>
 struct Scorer32 {
     static constexpr bool BLOCKS = true, BY_PLANE = true, WHOLE_WARPS = true;
-    static constexpr bool SMALL = ((2 * R) / ST + 1) * ((2 * R) / ST + 1) <= 25;
+    static constexpr PassForm FORM = F;
+    using Plane = PlaneF32;
     const ViewDesc* v;
     const float* s_ref;
-    Shared32<PX>& sm;
+    Shared32<PX, F>& sm;
     int x0, y0;
     __device__ __forceinline__ void begin(int lx, int ly) {
         sm.sums[threadIdx.x] = window_sums<R, ST>(s_ref, TILE_W + 2 * R, lx, ly);
     }
     __device__ __forceinline__ void publish() {}
-    __device__ __forceinline__ void set_plane(int k, int x, int y, float4 h, bool ok) {
-        const PlaneF32 p = plane_f32(v, x, y, h);
-        sm.plane[k] = make_float4(p.nK0, p.nK1, p.nK2, p.inv_n_dot_P);
-        sm.ok[k] = ok && p.ok;
+    __device__ __forceinline__ PlaneF32 plane(int x, int y, float4 h, bool ok) const {
+        PlaneF32 p = plane_f32(v, x, y, h);
+        p.ok = p.ok && ok;
+        return p;
     }
-    __device__ __forceinline__ float score(int s, int k, int o, int lx, int ly, bool live) const {
+    __device__ __forceinline__ bool has(const PlaneF32&) const { return true; }  // score's vote wants every lane
+    __device__ __forceinline__ void store(int k, const PlaneF32& p) {
+        sm.plane[k] = make_float4(p.nK0, p.nK1, p.nK2, p.inv_n_dot_P);
+        sm.ok[k] = p.ok;
+    }
+    __device__ __forceinline__ PlaneF32 load(int k) const {
         const float4 q = sm.plane[k];
-        return cost_f32<R, ST>(s_ref, TILE_W + 2 * R, lx, ly, x0 + lx, y0 + ly,
-                               PlaneF32{q.x, q.y, q.z, q.w, live && sm.ok[k] != 0}, sm.sums[o], v, s);
+        return PlaneF32{q.x, q.y, q.z, q.w, sm.ok[k] != 0};
+    }
+    __device__ __forceinline__ float score(int s, PlaneF32 p, int o, int lx, int ly, bool live) const {
+        p.ok = p.ok && live;
+        return cost_f32<R, ST>(s_ref, TILE_W + 2 * R, lx, ly, x0 + lx, y0 + ly, p, sm.sums[o], v, s);
     }
     __device__ __forceinline__ float mean(float sum, int k) const { return mean_f32(sum, k); }
 };
 
-template <int R, int ST, int TH>
+template <int R, int ST, int TH, PassForm F>
 __device__ __forceinline__ void tile_propagate(const ViewDesc* v, int x0, int y0, const SolveConsts& sc,
-                                               int iteration, int color, float* s_ref, Shared32<TILE_W * TH / 2>& sm,
-                                               bool roomy = false) {
+                                               int iteration, int color, float* s_ref,
+                                               Shared32<TILE_W * TH / 2, F>& sm) {
     constexpr int PX = TILE_W * TH / 2;
     load_ref_tile(s_ref, TILE_W + 2 * R, TH + 2 * R, v, x0, y0, R);
     __syncthreads();
-    Scorer32<R, ST, PX> scorer{v, s_ref, sm, x0, y0};
-    red_black_pass<CTA_THREADS, PX>(v, x0, y0, sc, iteration, color, scorer, sm.unit, sm.pass, roomy);
+    Scorer32<R, ST, PX, F> scorer{v, s_ref, sm, x0, y0};
+    red_black_pass<CTA_THREADS, PX>(v, x0, y0, sc, iteration, color, scorer, sm.unit, sm.pass);
 }
 
-template <int R, int ST, bool SPLIT>
-__global__ void __launch_bounds__(CTA_THREADS, pass_blocks<R, ST>()) propagate_kernel(BatchList bl,
-                                                                                         SolveConsts sc, int iteration,
-                                                                                         int color, bool roomy) {
-    constexpr int TH = SPLIT ? TILE_H / 2 : TILE_H;
+template <int R, int ST, PassForm F>
+__global__ void __launch_bounds__(CTA_THREADS, pass_blocks<R, ST, F>())
+    propagate_kernel(BatchList bl, SolveConsts sc, int iteration, int color) {
+    constexpr bool HALVES = F == PassForm::ROOMY || F == PassForm::SPLIT;
+    constexpr int TH = HALVES ? TILE_H / 2 : TILE_H;
     __shared__ float s_ref[(TILE_W + 2 * R) * (TH + 2 * R)];
-    __shared__ Shared32<TILE_W * TH / 2> sm;
+    __shared__ Shared32<TILE_W * TH / 2, F> sm;
     int tile_x, tile_y;
-    const ViewDesc* v = locate_tile(bl, SPLIT ? blockIdx.x >> 1 : blockIdx.x, &tile_x, &tile_y);
-    const int y0 = tile_y * TILE_H + (SPLIT ? (blockIdx.x & 1) * TH : 0);
-    tile_propagate<R, ST, TH>(v, tile_x * TILE_W, y0, sc, iteration, color, s_ref, sm, roomy);
+    const ViewDesc* v = locate_tile(bl, HALVES ? blockIdx.x >> 1 : blockIdx.x, &tile_x, &tile_y);
+    const int y0 = tile_y * TILE_H + (HALVES ? (blockIdx.x & 1) * TH : 0);
+    tile_propagate<R, ST, TH, F>(v, tile_x * TILE_W, y0, sc, iteration, color, s_ref, sm);
 }
 
 // Persistent form: one launch runs every stage of every view of a solve
 // (see Schedule), each CTA taking tiles until the tickets run out.  The stage
 // bodies are the functions the per-stage kernels above run, so the results
 // are bit-identical to the per-stage launch sequence.
-template <int R, int ST>
+template <int R, int ST, PassForm F>
 __global__ void __launch_bounds__(CTA_THREADS, PERSISTENT_BLOCKS) persistent_kernel(Schedule s) {
     __shared__ float s_ref[(TILE_W + 2 * R) * (TILE_H + 2 * R)];
-    __shared__ Shared32<CTA_THREADS> sm;
+    __shared__ Shared32<CTA_THREADS, F> sm;
     // The claimed tile lives in shared memory: warp 0 decodes it once and
     // thread 0 publishes it after the stage, so no thread carries it through the body.
     __shared__ SchedTile s_tile;
@@ -459,7 +475,7 @@ __global__ void __launch_bounds__(CTA_THREADS, PERSISTENT_BLOCKS) persistent_ker
             tile_cost<R, ST, TILE_H>(v, tx * TILE_W, ty * TILE_H, s.sc, s_ref);
         } else if (stage <= 2 * v->iterations) {
             const int k = stage - 1;
-            tile_propagate<R, ST, TILE_H>(v, tx * TILE_W, ty * TILE_H, s.sc, k >> 1, k & 1, s_ref, sm);
+            tile_propagate<R, ST, TILE_H, F>(v, tx * TILE_W, ty * TILE_H, s.sc, k >> 1, k & 1, s_ref, sm);
         } else if (is_filter_stage(v, stage)) {
             tile_filter(s.views, v, tx, ty, true);  // geometric check, then the maps
         } else {
@@ -473,16 +489,29 @@ __global__ void __launch_bounds__(CTA_THREADS, PERSISTENT_BLOCKS) persistent_ker
 template <int R, int ST>
 cudaError_t launch_rs(const BatchList& bl, const SolveConsts& sc, int iteration, int color, bool full,
                       cudaStream_t st) {
+    constexpr int N = window_taps(R, ST);
     const int tiles = bl.total_tiles, sms = device_sms();
-    if (split_tiles(tiles, sms)) {
-        if (full)
+    if (full) {
+        if (split_cost(tiles, sms))  // whole tiles -> halves, 701 x 439 (605 tiles), r 3 s 2, 6 sources: 152 -> 130 us
             cost_kernel<R, ST, true><<<2 * tiles, CTA_THREADS, 0, st>>>(bl, sc);
         else
-            propagate_kernel<R, ST, true><<<2 * tiles, CTA_THREADS, 0, st>>>(bl, sc, iteration, color, 2 * tiles <= 3 * sms);
-    } else if (full) {
-        cost_kernel<R, ST, false><<<tiles, CTA_THREADS, 0, st>>>(bl, sc);
-    } else {
-        propagate_kernel<R, ST, false><<<tiles, CTA_THREADS, 0, st>>>(bl, sc, iteration, color, false);
+            cost_kernel<R, ST, false><<<tiles, CTA_THREADS, 0, st>>>(bl, sc);
+        return cudaGetLastError();
+    }
+    switch (pass_form(PASS_RULE_F32, N, bl.max_sources, tiles, sms)) {
+        case PassForm::ROOMY:
+            propagate_kernel<R, ST, PassForm::ROOMY><<<2 * tiles, CTA_THREADS, 0, st>>>(bl, sc, iteration, color);
+            break;
+        case PassForm::SPLIT:
+            propagate_kernel<R, ST, PassForm::SPLIT><<<2 * tiles, CTA_THREADS, 0, st>>>(bl, sc, iteration, color);
+            break;
+        case PassForm::WHOLE:
+            if constexpr (N <= PASS_RULE_F32.whole)
+                propagate_kernel<R, ST, PassForm::WHOLE><<<tiles, CTA_THREADS, 0, st>>>(bl, sc, iteration, color);
+            break;
+        case PassForm::UNITS:
+            propagate_kernel<R, ST, PassForm::UNITS><<<tiles, CTA_THREADS, 0, st>>>(bl, sc, iteration, color);
+            break;
     }
     return cudaGetLastError();
 }
@@ -508,18 +537,27 @@ cudaError_t dispatch_f32(const BatchList& bl, const SolveConsts& sc, int iterati
 #undef HP_CASE
 }
 
-template <int R, int ST>
-cudaError_t persistent_rs(const Schedule& s, int grid, cudaStream_t st, int* occ) {
-    if (occ) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, persistent_kernel<R, ST>, CTA_THREADS, 0);
-    persistent_kernel<R, ST><<<grid, CTA_THREADS, 0, st>>>(s);
+template <int R, int ST, PassForm F>
+cudaError_t persistent_rsf(const Schedule& s, int grid, cudaStream_t st, int* occ) {
+    if (occ) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, persistent_kernel<R, ST, F>, CTA_THREADS, 0);
+    persistent_kernel<R, ST, F><<<grid, CTA_THREADS, 0, st>>>(s);
     return cudaGetLastError();
 }
 
-cudaError_t persistent_dispatch(int radius, int stride, const Schedule* s, int grid, cudaStream_t st, int* occ) {
+template <int R, int ST>
+cudaError_t persistent_rs(const Schedule& s, int grid, cudaStream_t st, int* occ) {
+    constexpr int N = window_taps(R, ST);
+    if constexpr (N <= PASS_RULE_F32.whole_persistent)
+        if (persistent_whole(PASS_RULE_F32, N, s.max_sources, s.tiles, device_sms()))
+            return persistent_rsf<R, ST, PassForm::WHOLE>(s, grid, st, occ);
+    return persistent_rsf<R, ST, PassForm::UNITS>(s, grid, st, occ);
+}
+
+cudaError_t persistent_dispatch(int radius, int stride, const Schedule& s, int grid, cudaStream_t st, int* occ) {
     if (stride != 1 && stride != 2) return cudaErrorInvalidValue;
-#define HP_CASE(RR)                                                                              \
-    case RR:                                                                                     \
-        return stride == 1 ? persistent_rs<RR, 1>(*s, grid, st, occ) : persistent_rs<RR, 2>(*s, grid, st, occ);
+#define HP_CASE(RR) \
+    case RR:        \
+        return stride == 1 ? persistent_rs<RR, 1>(s, grid, st, occ) : persistent_rs<RR, 2>(s, grid, st, occ);
     switch (radius) {
         HP_CASE(1)
         HP_CASE(2)
@@ -539,12 +577,14 @@ cudaError_t launch_persistent_f32(const Schedule& s, int grid, cudaStream_t st) 
     if (s.total <= 0 || grid <= 0) return cudaSuccess;
     Schedule k = s;
     if (!k.abort) k.abort = k.status + 1;
-    return persistent_dispatch(k.sc.radius, k.sc.stride, &k, grid, st, nullptr);
+    return persistent_dispatch(k.sc.radius, k.sc.stride, k, grid, st, nullptr);
 }
 
-cudaError_t persistent_occupancy_f32(int radius, int stride, int* blocks_per_sm) {
-    Schedule dummy{};
-    return persistent_dispatch(radius, stride, &dummy, 0, nullptr, blocks_per_sm);
+cudaError_t persistent_occupancy_f32(const SolveConsts& sc, int tiles, int max_sources, int* blocks_per_sm) {
+    Schedule s{};
+    s.tiles = tiles;
+    s.max_sources = max_sources;
+    return persistent_dispatch(sc.radius, sc.stride, s, 0, nullptr, blocks_per_sm);
 }
 
 cudaError_t launch_init(const BatchList& bl, int tile_h, cudaStream_t st) {

@@ -62,7 +62,7 @@ struct hp_plan {
     int* d_done = nullptr;
     size_t done_bytes = 0;
     int* d_lists = nullptr;
-    std::vector<int> list_off, list_count, list_tiles;
+    std::vector<int> list_off, list_count, list_tiles, list_sources;
     int* d_entry_ticket = nullptr;
     int2* d_entry_info = nullptr;
     int n_entries = 0, total = 0;
@@ -129,6 +129,8 @@ hp::Schedule schedule_of(const hp_plan* p) {
     s.stall_view = p->opt.debug_stall_view;
     s.stall_tile = p->opt.debug_stall_view >= 0 ? p->opt.debug_stall_tile : -1;
     s.sc = plan_consts(p);
+    s.tiles = p->list_tiles[0];
+    s.max_sources = p->list_sources[0];
     s.main_done = p->filter_order.empty() ? nullptr : p->d_counter + 4;
     s.main_total = p->filter_order.empty() ? p->total : p->main_total;
     return s;
@@ -141,6 +143,7 @@ hp::BatchList list_of(const hp_plan* p, int l) {
     bl.active = p->d_lists + p->list_off[l];
     bl.tile_prefix = bl.active + bl.n_active;
     bl.total_tiles = p->list_tiles[l];
+    bl.max_sources = p->list_sources[l];
     return bl;
 }
 
@@ -298,8 +301,8 @@ hp_status plan_occupancy(hp_plan* p) {
     hp_ctx* ctx = p->ctx;
     const hp::SolveConsts sc = plan_consts(p);
     HP_CUDA(p->params.precision == HP_PRECISION_F16ACC
-                ? hp::persistent_occupancy_f16(sc, &p->occ)
-                : hp::persistent_occupancy_f32(p->params.radius, p->params.stride, &p->occ));
+                ? hp::persistent_occupancy_f16(sc, p->list_tiles[0], p->list_sources[0], &p->occ)
+                : hp::persistent_occupancy_f32(sc, p->list_tiles[0], p->list_sources[0], &p->occ));
     if (p->occ < 1) return fail(ctx, HP_ERR_UNSUPPORTED, "plan: persistent kernel does not fit on an SM");
     return HP_OK;
 }
@@ -324,6 +327,7 @@ hp_status build_device(hp_plan* p, int tile_h) {
     p->list_off.clear();
     p->list_count.clear();
     p->list_tiles.clear();
+    p->list_sources.clear();
     for (int k = 0; k < num_jobs; ++k) {
         if ((st = fill_desc(ctx, &jobs[k], k, &p->host[k], tile_h)) != HP_OK) return st;
         p->iters.push_back(jobs[k].iterations);
@@ -346,6 +350,9 @@ hp_status build_device(hp_plan* p, int tile_h) {
         }
         ints.push_back(acc);
         p->list_tiles.push_back(acc);
+        int sources = 0;
+        for (int k : act) sources = std::max(sources, p->host[k].S);
+        p->list_sources.push_back(sources);
     }
     // Geometric-consistency stages (hp_params.filter_*).
     std::vector<hp::FilterStage> fstages;

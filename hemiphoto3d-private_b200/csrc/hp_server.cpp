@@ -470,6 +470,11 @@ bool enqueue_step(hp_server* s) {
                     sch.stall_tile = s->opt.debug_stall_tile;
                 }
         sch.sc = s->sc;
+        for (CoreReq* c : sp.reqs) {
+            const hp::ViewDesc& d = static_cast<SrvReq*>(c->user)->desc;
+            sch.tiles += d.tiles_x * d.tiles_y;
+            sch.max_sources = std::max(sch.max_sources, d.S);
+        }
         const int grid = std::max(1, std::min(totals[l], s->sms * s->cpsm));
         e = f16 ? hp::launch_persistent_f16(sch, grid, s->stream) : hp::launch_persistent_f32(sch, grid, s->stream);
         if (e == cudaSuccess)
@@ -783,8 +788,8 @@ hp_status hp_server_create(hp_ctx* ctx, const hp_params* params, const hp_server
     uint64_t keep = ~0ull;  // keep freed state cached for the next requests
     HP_CUDA(cudaMemPoolSetAttribute(s->pool, cudaMemPoolAttrReleaseThreshold, &keep));
     HP_CUDA(cudaDeviceGetAttribute(&s->sms, cudaDevAttrMultiProcessorCount, ctx->device));
-    HP_CUDA(params->precision == HP_PRECISION_F16ACC ? hp::persistent_occupancy_f16(s->sc, &s->occ)
-                                                     : hp::persistent_occupancy_f32(params->radius, params->stride, &s->occ));
+    HP_CUDA(params->precision == HP_PRECISION_F16ACC ? hp::persistent_occupancy_f16(s->sc, 0, HP_MAX_SOURCES, &s->occ)
+                                                     : hp::persistent_occupancy_f32(s->sc, 0, HP_MAX_SOURCES, &s->occ));
     if (s->occ < 1) return fail(ctx, HP_ERR_UNSUPPORTED, "server_create: persistent kernel does not fit on an SM");
     s->cpsm = (o.ctas_per_sm > 0 && o.ctas_per_sm < s->occ) ? o.ctas_per_sm : s->occ;
     size_t fr = 0;

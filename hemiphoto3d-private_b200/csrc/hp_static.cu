@@ -187,6 +187,7 @@ extern "C" hp_status hp_solve_static(int device, void* stream, const hp_job* job
     bl.tile_prefix = bl.active + 1;
     bl.n_active = 1;
     bl.total_tiles = list[2];
+    bl.max_sources = d.S;
     hp::SolveConsts sc;
     sc.radius = params->radius;
     sc.stride = params->stride;
