@@ -53,11 +53,18 @@ template <int R, int ST, PassForm F>
 constexpr int pass_blocks() {
     return F == PassForm::ROOMY || F == PassForm::WHOLE || (2 * R) / ST + 1 > 8 ? 3 : 4;
 }
-// Persistent launches: a small batch has fewer tiles at a stage than three CTAs
-// an SM, and the surplus CTAs wait on dependencies where others would run.  With
-// 2 and with pass_blocks(): 3 views up to 457 x 279, r 7, s 1, 5131 us and 7453;
-// 3 up to 320 x 240, r 3, s 2, 1176 and 1775; 3 up to 869 x 565 43.2 and 42.8 ms.
-constexpr int PERSISTENT_BLOCKS = 2;
+// Persistent launches of few tiles take two CTAs an SM: beyond the tiles that can run at
+// a time, CTAs wait on dependencies where others would run, and a CTA that runs has the
+// registers.  With many tiles all of pass_blocks() pay, from 4 tiles an SM (of all views
+// together) for rows of up to 8 taps, from 8 for longer ones.  2 CTAs -> pass_blocks():
+//  r 7 s 2, 6 sources, 5 iterations: 3 x 320 x 240 (3.0 tiles an SM) 2860 -> 3428 us, 3 x
+//   457 x 279 (5.7) 4928 -> 4475, 4 x 1920 x 1080 (109) 116.3 -> 103.7 ms;
+//  r 5 s 1, 4 sources: 5.7 tiles an SM 5446 -> 5468 us, 8.9 8784 -> 8611, 109 133.4 -> 128.0 ms;
+//  r 3 s 2, 3 sources (items whole): 1.0 486 -> 705 us, 3.0 660 -> 595, 109 25.3 -> 20.3 ms.
+template <int R, int ST>
+constexpr int many_tiles() { return (2 * R) / ST + 1 <= 8 ? 4 : 8; }
+template <int R, int ST, PassForm F, bool MANY>
+constexpr int persistent_blocks() { return MANY ? pass_blocks<R, ST, F>() : 2; }
 constexpr int COST_BLOCKS = 3;  // full-map cost, 1920 x 1080, r 5, s 1: 1486 us, 1574 with 2, 1506 with 4
 
 // Locate the view and tile of this CTA in a batch launch.
@@ -449,8 +456,8 @@ __global__ void __launch_bounds__(CTA_THREADS, pass_blocks<R, ST, F>())
 // (see Schedule), each CTA taking tiles until the tickets run out.  The stage
 // bodies are the functions the per-stage kernels above run, so the results
 // are bit-identical to the per-stage launch sequence.
-template <int R, int ST, PassForm F>
-__global__ void __launch_bounds__(CTA_THREADS, PERSISTENT_BLOCKS) persistent_kernel(Schedule s) {
+template <int R, int ST, PassForm F, bool MANY>
+__global__ void __launch_bounds__(CTA_THREADS, persistent_blocks<R, ST, F, MANY>()) persistent_kernel(Schedule s) {
     __shared__ float s_ref[(TILE_W + 2 * R) * (TILE_H + 2 * R)];
     __shared__ Shared32<CTA_THREADS, F> sm;
     // The claimed tile lives in shared memory: warp 0 decodes it once and
@@ -539,8 +546,10 @@ cudaError_t dispatch_f32(const BatchList& bl, const SolveConsts& sc, int iterati
 
 template <int R, int ST, PassForm F>
 cudaError_t persistent_rsf(const Schedule& s, int grid, cudaStream_t st, int* occ) {
-    if (occ) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, persistent_kernel<R, ST, F>, CTA_THREADS, 0);
-    persistent_kernel<R, ST, F><<<grid, CTA_THREADS, 0, st>>>(s);
+    const bool many = s.tiles > many_tiles<R, ST>() * device_sms();
+    const auto kernel = many ? persistent_kernel<R, ST, F, true> : persistent_kernel<R, ST, F, false>;
+    if (occ) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, kernel, CTA_THREADS, 0);
+    kernel<<<grid, CTA_THREADS, 0, st>>>(s);
     return cudaGetLastError();
 }
 

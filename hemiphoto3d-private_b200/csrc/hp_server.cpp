@@ -184,7 +184,7 @@ struct hp_server {
     hp::SolveConsts sc{};
     cudaStream_t stream = nullptr;
     cudaMemPool_t pool = nullptr;
-    int sms = 0, occ = 0, cpsm = 1;
+    int sms = 0;
     size_t total_mem = 0;
     size_t ring_bytes = 0;
     int max_launches = 1;
@@ -475,8 +475,13 @@ bool enqueue_step(hp_server* s) {
             sch.tiles += d.tiles_x * d.tiles_y;
             sch.max_sources = std::max(sch.max_sources, d.S);
         }
-        const int grid = std::max(1, std::min(totals[l], s->sms * s->cpsm));
-        e = f16 ? hp::launch_persistent_f16(sch, grid, s->stream) : hp::launch_persistent_f32(sch, grid, s->stream);
+        int occ = 1;  // of the kernel that this step's views take
+        e = f16 ? hp::persistent_occupancy_f16(sch.sc, sch.tiles, sch.max_sources, &occ)
+                : hp::persistent_occupancy_f32(sch.sc, sch.tiles, sch.max_sources, &occ);
+        const int cpsm = s->opt.ctas_per_sm > 0 ? std::min(s->opt.ctas_per_sm, occ) : occ;
+        const int grid = std::max(1, std::min(totals[l], s->sms * cpsm));
+        if (e == cudaSuccess)
+            e = f16 ? hp::launch_persistent_f16(sch, grid, s->stream) : hp::launch_persistent_f32(sch, grid, s->stream);
         if (e == cudaSuccess)
             e = cudaMemcpyAsync(slot.host_status + 4 * l, sch.status, 3 * sizeof(int), cudaMemcpyDeviceToHost,
                                 s->stream);
@@ -788,10 +793,10 @@ hp_status hp_server_create(hp_ctx* ctx, const hp_params* params, const hp_server
     uint64_t keep = ~0ull;  // keep freed state cached for the next requests
     HP_CUDA(cudaMemPoolSetAttribute(s->pool, cudaMemPoolAttrReleaseThreshold, &keep));
     HP_CUDA(cudaDeviceGetAttribute(&s->sms, cudaDevAttrMultiProcessorCount, ctx->device));
-    HP_CUDA(params->precision == HP_PRECISION_F16ACC ? hp::persistent_occupancy_f16(s->sc, 0, HP_MAX_SOURCES, &s->occ)
-                                                     : hp::persistent_occupancy_f32(s->sc, 0, HP_MAX_SOURCES, &s->occ));
-    if (s->occ < 1) return fail(ctx, HP_ERR_UNSUPPORTED, "server_create: persistent kernel does not fit on an SM");
-    s->cpsm = (o.ctas_per_sm > 0 && o.ctas_per_sm < s->occ) ? o.ctas_per_sm : s->occ;
+    int occ = 0;
+    HP_CUDA(params->precision == HP_PRECISION_F16ACC ? hp::persistent_occupancy_f16(s->sc, 0, HP_MAX_SOURCES, &occ)
+                                                     : hp::persistent_occupancy_f32(s->sc, 0, HP_MAX_SOURCES, &occ));
+    if (occ < 1) return fail(ctx, HP_ERR_UNSUPPORTED, "server_create: persistent kernel does not fit on an SM");
     size_t fr = 0;
     HP_CUDA(cudaMemGetInfo(&fr, &s->total_mem));
     // Upload area of one step: max_active descriptors, and per launch its counters and a

@@ -118,3 +118,28 @@ def test_solve_equals_its_half_passes_where_smaller_launches_end(hp, scene_mod, 
             for color in (0, 1):
                 ctx.propagate_pass(job, params, maps, it, color)
     assert np.array_equal(d, d2) and np.array_equal(n, n2) and np.array_equal(c, c2)
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("radius,stride,sources", [(1, 1, 3), (3, 2, 4), (4, 2, 3), (5, 1, 2), (7, 2, 6), (7, 1, 2)])
+def test_persistent_launches_of_many_tiles(hp, small, precision, radius, stride, sources):
+    """Past 8 tiles an SM, persistent launches take their kernels for many tiles: plan and server."""
+    s, ctx, ids = small
+    k = 8 * _sms() // TILES + 1
+    assert TILES * k > 8 * _sms()
+    params = hp.default_params(radius=radius, stride=stride, precision=precision)
+    job = _job(hp, s, ids, 4, sources, 3)
+    maps, d, n, c = hp.host_maps(H, W)
+    ctx.solve([job], params, [maps])
+    outs = [hp.host_maps(H, W) for _ in range(k)]
+    with hp.Plan(ctx, [job] * k, params, [o[0] for o in outs],
+                 hp.plan_options(schedule=hp.SCHEDULE_PERSISTENT)) as plan:
+        plan.run()
+    served = [hp.host_maps(H, W) for _ in range(k)]
+    with hp.Server(ctx, params) as server:
+        for o in served:
+            server.submit(job, o[0])
+        server.drain()
+        server.poll()
+    for _, a, b, e in outs + served:
+        assert np.array_equal(a, d) and np.array_equal(b, n) and np.array_equal(e, c)
