@@ -941,7 +941,7 @@ hp_status hp_fuse_depth_maps(hp_ctx* ctx, const hp_fuse_view* views, int num_vie
     size_t staged_floats = 0;
     for (int i = 0; i < num_views; ++i)
         if (views[i].width > 0 && views[i].height > 0) pixels += static_cast<long long>(views[i].width) * views[i].height;
-    const int steps = hp::fuse_steps(pixels), cta_px = steps * hp::FUSE_THREADS;
+    const int steps = hp::fuse_steps(pixels, hp::device_sms()), cta_px = steps * hp::FUSE_THREADS;
     for (int i = 0; i < num_views; ++i) {
         const hp_fuse_view& v = views[i];
         if (v.width < 1 || v.height < 1 || v.width > 65536 || v.height > 65536)

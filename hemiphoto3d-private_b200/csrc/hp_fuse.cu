@@ -198,7 +198,6 @@ __device__ __forceinline__ Fused fuse_pixel(const FuseArgs& a, int i, int x, int
 }
 
 constexpr int STEP_WORDS = FUSE_THREADS / 32;  // ballot words per step
-constexpr int FUSE_BLOCKS = 6;                // resident CTAs per SM the passes are register-budgeted for
 
 __global__ void __launch_bounds__(FUSE_THREADS, FUSE_BLOCKS) fuse_count_kernel(FuseArgs a, unsigned* ballots,
                                                                                int* block_counts) {

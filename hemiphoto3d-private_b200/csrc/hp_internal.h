@@ -270,13 +270,17 @@ struct FuseArgs {
     float min_conf, max_depth_rel, max_reproj_sq, min_normal_cos;
 };
 constexpr int FUSE_THREADS = 256;
+constexpr int FUSE_BLOCKS = 6;  // resident CTAs per SM the fusion passes are register-budgeted for
 // Steps of FUSE_THREADS pixels a CTA of the fusion kernels takes.  Four give the
 // writing pass full warps where a third of the pixels emit; with one, small
-// inputs fill the GPU (4 views of 279 x 210: 111 us with four, 79 with one and
-// the kept workspace).  The line is two waves of four-step CTAs.
+// inputs fill the GPU.  The line is two waves of four-step CTAs (1.8 Mpx on 148
+// SMs).  Whole call on device maps, the workspace kept, one step / four: 8 x 279 x
+// 210 (0.5 Mpx) 108 / 144 us, 8 x 400 x 300 (1.0) 135 / 159, 3 x 961 x 541 (1.6)
+// 127 / 125, 8 x 560 x 420 (1.9) 191 / 194, 5 x 800 x 600 (2.4) 196 / 177, 8 x 1921
+// x 1081 (16.6) 1227 / 1027.
 constexpr int FUSE_STEPS = 4;
-inline int fuse_steps(long long pixels) {
-    return pixels >= 2ll * 148 * 6 * FUSE_STEPS * FUSE_THREADS ? FUSE_STEPS : 1;
+inline int fuse_steps(long long pixels, int sms) {
+    return pixels >= 2ll * sms * FUSE_BLOCKS * FUSE_STEPS * FUSE_THREADS ? FUSE_STEPS : 1;
 }
 
 }  // namespace hp
