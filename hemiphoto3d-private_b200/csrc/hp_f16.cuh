@@ -624,10 +624,12 @@ __global__ void __launch_bounds__(Tile<TH>::NT, Tile<TH>::MIN_BLOCKS) cost16_ker
 
 // Scorer of the half-pass (red_black_pass): a unit reads its pixel's window
 // statistics and s_win column, and its item's plane vector, from shared memory.
-template <int R, int ST, int TH, int D, int NT, PassForm F>
+template <int R, int ST, int TH, int D, int NT, PassForm F, bool PERSISTENT>
 struct Scorer16 {
     static constexpr int PX = 32 * TH, TW = TILE_W + 2 * R;
     static constexpr bool BLOCKS = !Win<R, ST>::IN_SMEM, BY_PLANE = false, WHOLE_WARPS = false;
+    static constexpr bool EAGER = PERSISTENT || F != PassForm::UNITS || !Win<R, ST>::IN_SMEM ||
+                                  Win<R, ST>::SIDE * Win<R, ST>::VEC < 28;
     static constexpr PassForm FORM = F;
     using Plane = float4;
     const ViewDesc* v;
@@ -653,12 +655,12 @@ struct Scorer16 {
     __device__ __forceinline__ float mean(float sum, int k) const { return __fdiv_rn(sum, static_cast<float>(k)); }
 };
 
-template <int R, int ST, int TH, int D, int NT, PassForm F>
+template <int R, int ST, int TH, int D, bool PERSISTENT, int NT, PassForm F>
 __device__ __forceinline__ void tile_propagate16(const ViewDesc* v, int x0, int y0, const SolveConsts& sc,
                                                  int iteration, int color, Shared<R, ST, TH, NT, F>& sm) {
     load_ref_tile16<NT>(sm.ref, TILE_W + 2 * R, TH + 2 * R, v, x0, y0, R);
     __syncthreads();
-    Scorer16<R, ST, TH, D, NT, F> scorer{v, sm, x0, y0, sc.soft_mask};
+    Scorer16<R, ST, TH, D, NT, F, PERSISTENT> scorer{v, sm, x0, y0, sc.soft_mask};
     red_black_pass<NT, 32 * TH>(v, x0, y0, sc, iteration, color, scorer, sm.units(), sm.pass);
 }
 
@@ -676,7 +678,8 @@ __global__ void __launch_bounds__(Tile<TH>::NT, Tile<TH>::MIN_BLOCKS) propagate1
     int tile_x, tile_y;
     const ViewDesc* v = locate_tile16(bl, P::HALVES ? blockIdx.x >> 1 : blockIdx.x, &tile_x, &tile_y);
     const int y0 = tile_y * TH + (P::HALVES ? (blockIdx.x & 1) * P::ROWS : 0);
-    tile_propagate16<R, ST, P::ROWS, D>(v, tile_x * TILE_W, y0, sc, iteration, color, shared_of<typename P::Smem>());
+    tile_propagate16<R, ST, P::ROWS, D, false>(v, tile_x * TILE_W, y0, sc, iteration, color,
+                                               shared_of<typename P::Smem>());
 }
 
 // Persistent form (see Schedule and the FP32 persistent kernel): the stage
@@ -720,7 +723,7 @@ __global__ void __launch_bounds__(Tile<TH>::NT, Tile<TH>::MIN_BLOCKS) persistent
             tile_cost16<R, ST, TH, D>(v, tx, ty, s.sc, sm);
         } else if (stage <= 2 * v->iterations) {
             const int k = stage - 1;
-            tile_propagate16<R, ST, TH, D>(v, tx * TILE_W, ty * TH, s.sc, k >> 1, k & 1, sm);
+            tile_propagate16<R, ST, TH, D, true>(v, tx * TILE_W, ty * TH, s.sc, k >> 1, k & 1, sm);
         } else if (is_filter_stage(v, stage)) {
             tile_filter(s.views, v, tx, ty, true);  // geometric check, then the maps
         } else {
@@ -785,7 +788,7 @@ struct Dispatch {
             if (form == PassForm::ROOMY) return pass<R, ST, 4, PassForm::ROOMY>(*bl, sc, iteration, color, st);
             if (form == PassForm::SPLIT) return pass<R, ST, 4, PassForm::SPLIT>(*bl, sc, iteration, color, st);
         }
-        // Units earn their keep by the trial bound; a half-pass on caller maps goes without it (1921 x 1081, whole call,
+        // Units earn their keep by the trial bound; a half-pass on caller maps goes without it (1921 x 1081, the call,
         // units -> whole: r 7 s 2, 6 sources 3329 -> 3201 us, 1 source 692 -> 641; r 1 s 1, 6 sources 941 -> 783).
         if (form == PassForm::WHOLE || !sc.memo)
             return pass<R, ST, 4, PassForm::WHOLE>(*bl, sc, iteration, color, st);

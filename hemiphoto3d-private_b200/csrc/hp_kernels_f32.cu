@@ -396,7 +396,7 @@ struct Shared32 {
 // Scorer of the half-pass (red_black_pass).
 template <int R, int ST, int PX, PassForm F>
 struct Scorer32 {
-    static constexpr bool BLOCKS = true, BY_PLANE = true, WHOLE_WARPS = true;
+    static constexpr bool BLOCKS = true, BY_PLANE = true, WHOLE_WARPS = true, EAGER = true;
     static constexpr PassForm FORM = F;
     using Plane = PlaneF32;
     const ViewDesc* v;

@@ -117,6 +117,7 @@ __device__ __forceinline__ int pass_thread(int lx, int ly) {
 //                               that are not live take part for their warp's sake
 //   mean(sum, k)                sum / k, monotone in sum
 //   BLOCKS                      pass_pixel's layout
+//   EAGER                       neighbour_needs' order of reads
 //   BY_PLANE                    neighbour items are listed by the plane they score, not by pixel
 //   FORM                        the launch's PassForm
 //   WHOLE_WARPS                 score starts with a vote of all 32 lanes of a warp
@@ -140,7 +141,7 @@ __device__ __forceinline__ void red_black_pass(const ViewDesc* v, int x0, int y0
         scorer.begin(lx, ly);
         best = v->hyp[idx];
         best_cost = sc.memo ? cost_value(v->cost[idx]) : v->cost[idx];  // a caller's cost as it is
-        need = neighbour_needs(v, x, y, best, sc.memo && iteration > 0);
+        need = neighbour_needs<K::EAGER>(v, x, y, best, sc.memo && iteration > 0);
     }
     scorer.publish();
     // Neighbour items are listed by pixel (bit 4 + c of `list`: the own pixel's neighbour c), or by plane: thread t

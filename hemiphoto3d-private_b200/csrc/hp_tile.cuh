@@ -73,6 +73,18 @@ __device__ __forceinline__ bool same_plane(float4 a, float4 b) {
 // On 1920 x 1080, r 7, s 2, 6 sources, 12 iterations this leaves 1.54 of the
 // 1.78 planes per visit the identity rule alone leaves (3000 x 2000 with noise,
 // 8 sources: 1.53 of 1.94).
+//
+// Settled neighbours' planes are read for those identity tests only, so a pixel
+// could read the costs first and then, mostly, no plane at all.  That is two round
+// trips in a row, which small launches and small windows pay in full: EAGER fetches
+// all planes and costs at once, then decides (planes after costs -> at once: FP32
+// 253 x 175, r 1 s 1, 1 source, 6 iterations 253 -> 228 us; 1920 x 1080, 12
+// iterations, r 1 s 1, 1 source FP32 4.87 -> 4.18 ms, FP16-acc r 5 s 2, 4 sources
+// 17.25 -> 16.58; FP16-acc plans of 4 x 1920 x 1080, r 7 s 2, 6 sources 135.6 ->
+// 133.1).  Per-pass FP16-acc launches in units with wide rows in shared memory have
+// little L1 left for the planes and read them late (1920 x 1080, 6 sources, r 7 s 2
+// 34.4 ms, at once 35.3; r 3 s 1 27.3 and 28.1).
+template <bool EAGER>
 __device__ __forceinline__ unsigned neighbour_needs(const ViewDesc* v, int x, int y, float4 own, bool memo) {
     const int W = v->W, H = v->H;
     const float dmin = v->dmin, dmax = v->dmax;
@@ -81,22 +93,35 @@ __device__ __forceinline__ unsigned neighbour_needs(const ViewDesc* v, int x, in
         return static_cast<size_t>(y + (cand == 2 ? -1 : (cand == 3 ? 1 : 0))) * W + x +
                (cand == 0 ? -1 : (cand == 1 ? 1 : 0));
     };
+    float4 h[4];
+    float c[4];
 #pragma unroll
     for (int cand = 0; cand < 4; ++cand) {
+        h[cand] = make_float4(0.f, 0.f, 0.f, 0.f);
+        c[cand] = 0.f;
         const bool inside = cand == 0 ? x > 0 : (cand == 1 ? x + 1 < W : (cand == 2 ? y > 0 : y + 1 < H));
         if (inside) {
             need |= 1u << cand;
-            if (memo && cost_settled(v->cost[at(cand)])) settled |= 1u << cand;
+            if (memo) c[cand] = v->cost[at(cand)];
+            if constexpr (EAGER) h[cand] = v->hyp[at(cand)];
         }
     }
+#pragma unroll
+    for (int cand = 0; cand < 4; ++cand)
+        if (cost_settled(c[cand])) settled |= 1u << cand;
     need &= ~settled;
+    auto plane = [&](int cand) {
+        if constexpr (EAGER) return h[cand];
+        return v->hyp[at(cand)];
+    };
 #pragma unroll
     for (int cand = 0; cand < 4; ++cand) {
         if (!(need & (1u << cand))) continue;
-        const float4 h = v->hyp[at(cand)];
-        bool drop = h.x < dmin || h.x > dmax || same_plane(h, own);
-        for (int j = 0; j < 4 && !drop; ++j)
-            if (((j < cand ? need : 0u) | settled) & (1u << j)) drop = same_plane(h, v->hyp[at(j)]);
+        const float4 p = plane(cand);
+        bool drop = p.x < dmin || p.x > dmax || same_plane(p, own);
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (!drop && j != cand && (((j < cand ? need : 0u) | settled) & (1u << j))) drop = same_plane(p, plane(j));
         if (drop) need &= ~(1u << cand);
     }
     return need;
