@@ -108,22 +108,33 @@ constexpr int window_taps(int radius, int stride) { return ((2 * radius) / strid
 //   sources 2398 -> 2285; r 3 s 2, 3 sources 1923 -> 1845; 1921 x 1081, r 3 s 1, 3
 //   sources (147) 11100 units, 12345 whole.  FP32 573 x 303: r 1 s 1, 1 source
 //   377 -> 342; r 3 s 2, 2 sources (32) 575 units, 563 whole.
-//  split, S >= 3 / S < 3: tiles an SM up to which half tiles win.  FP16-acc, units ->
-//   halves: r 3 s 1, 3 sources (147) 2.3 tiles an SM 1232 -> 1199, 5.1 2036 -> 2127;
-//   r 7 s 2, 8 sources (512) 4.5 5206 -> 4896, 7.4 7732 -> 7660; 2 sources (128) 2.1
-//   1235 -> 1195, 2.3 1169 -> 1234.  FP32: r 5 s 2, 3 sources (108) 4.5 1925 -> 1891,
-//   6.1 2385 -> 2408; r 7 s 2, 2 sources (128) 2.1 1291 -> 1322; r 5 s 1, 2 sources
-//   (242) 2.3 2610 -> 2426, 3.1 2880 -> 2930.
+//  split: tiles an SM up to which half tiles win, units -> halves there and past it.
+//   FP16-acc, one or two sources 2.2: r 7 s 2, 2 sources (128) 2.1 tiles an SM 1235 ->
+//   1195, 2.3 1169 -> 1234; r 5 s 1, 1 source (121) 2.1 1145 -> 1051, 4.5 1633 -> 1693.
+//   More sources, by samples x sources / 175: r 3 s 1, 3 sources (147) 2.3 1232 -> 1199,
+//   5.1 2036 -> 2127; r 2 s 1, 8 iterations, 6 sources (150) 4.4 2660 -> 2549; r 5 s 2, 5
+//   sources (180) 4.5 2475 -> 2395, 5.4 2713 -> 2861; r 7 s 2, 8 sources (512) 4.5 5206
+//   -> 4896, 7.4 7732 -> 7660.
+//   FP32, two sources by samples / 100 (a part of one source gives half the threads of a
+//   half tile a unit): r 7 s 2 (128) 2.1 1291 -> 1322; r 5 s 1 (242) 2.3 2610 -> 2426, 3.1
+//   2880 -> 2930.  Others by samples / 24: r 5 s 2, 3 sources (108) 4.5 1925 -> 1891, 6.1
+//   2385 -> 2408; r 5 s 1, 1 source (121) 4.5 2076 -> 2038, 5.1 2335 -> 2390.
 //  A single half-pass on caller maps has no trial bound, so units gain by halves alone:
 //   FP16-acc 641 x 479 (4.1 tiles an SM), r 7 s 2, 3 sources 323 whole, 306 halves.
 struct PassRule {
-    int whole, whole_persistent;  // WHOLE up to so many samples, in per-pass and in persistent launches
-    int many, few;                // SPLIT up to samples / many (three or more sources) or samples / few tiles an SM,
-    float many_max, few_max;      // and up to these
+    int whole, whole_persistent;                 // WHOLE up to so many samples, per-pass and persistent launches
+    float (*split_up_to)(int samples, int sources);  // SPLIT up to so many tiles an SM
 };
-constexpr PassRule PASS_RULE_F32{27, 64, 24, 100, 8.0f, 8.0f};
-constexpr PassRule PASS_RULE_F16{100, 100, 50, 100, 8.0f, 2.25f};
-constexpr PassRule PASS_RULE_F16_SINGLE{100, 100, 25, 30, 5.0f, 5.0f};
+inline float split_f32(int samples, int sources) { return std::min(8.0f, samples / (sources == 2 ? 100.0f : 24.0f)); }
+inline float split_f16(int samples, int sources) {
+    return sources < 3 ? 2.2f : std::min(8.0f, std::max(2.2f, samples * sources / 175.0f));
+}
+inline float split_f16_single(int samples, int sources) {
+    return std::min(5.0f, samples / (sources < 3 ? 30.0f : 25.0f));
+}
+constexpr PassRule PASS_RULE_F32{27, 64, split_f32};
+constexpr PassRule PASS_RULE_F16{100, 100, split_f16};
+constexpr PassRule PASS_RULE_F16_SINGLE{100, 100, split_f16_single};
 inline bool roomy_tiles(int tiles, int sms) { return 2 * tiles <= 3 * sms; }
 inline bool halves_spread(int tiles, int sms) { return tiles % sms > 0 && 2 * (tiles % sms) <= sms; }
 inline bool split_cost(int tiles, int sms) { return tiles <= sms || (tiles <= 8 * sms && halves_spread(tiles, sms)); }
@@ -138,9 +149,7 @@ inline PassForm pass_form(const PassRule& r, int taps, int max_sources, int tile
     const int samples = taps * max_sources;
     if (roomy_tiles(tiles, sms)) return PassForm::ROOMY;
     if (samples <= r.whole) return PassForm::WHOLE;
-    const float most = max_sources >= 3 ? std::min(r.many_max, static_cast<float>(samples) / r.many)
-                                        : std::min(r.few_max, static_cast<float>(samples) / r.few);
-    return halves_spread(tiles, sms) && tiles <= most * sms ? PassForm::SPLIT : PassForm::UNITS;
+    return halves_spread(tiles, sms) && tiles <= r.split_up_to(samples, max_sources) * sms ? PassForm::SPLIT : PassForm::UNITS;
 }
 inline int device_sms() {
     int dev = 0, sms = 148;

@@ -17,7 +17,7 @@ pytestmark = pytest.mark.gpu
 
 W, H = 203, 130  # 4 x 17 tiles; the last row of tiles has two rows of pixels, so its lower halves none
 TILES = 4 * 17
-RULE = {0: (27, 24, 100, 8.0, 8.0), 1: (100, 50, 100, 8.0, 2.25)}  # precision: whole, many, few, maxima
+WHOLE_SAMPLES = {0: 27, 1: 100}  # by precision
 
 
 def _sms():
@@ -26,13 +26,15 @@ def _sms():
 
 
 def _form(precision, radius, stride, sources, tiles, sms):
-    whole, many, few, many_max, few_max = RULE[precision]
     samples = ((2 * radius) // stride + 1) ** 2 * sources
     if 2 * tiles <= 3 * sms:
         return "roomy"
-    if samples <= whole:
+    if samples <= WHOLE_SAMPLES[precision]:
         return "whole"
-    most = min(many_max, samples / many) if sources >= 3 else min(few_max, samples / few)
+    if precision == 0:
+        most = min(8, samples / (100 if sources == 2 else 24))
+    else:
+        most = 2.2 if sources < 3 else min(8, max(2.2, samples * sources / 175))
     past = tiles % sms
     return "split" if 0 < 2 * past <= sms and tiles <= most * sms else "units"
 
@@ -103,7 +105,7 @@ def test_solve_equals_its_half_passes_where_smaller_launches_end(hp, scene_mod, 
     form = _form(precision, radius, stride, sources, tiles, sms)
     if sms == 148:  # 234 tiles spread no better in halves, 342 do
         samples = ((2 * radius) // stride + 1) ** 2 * sources
-        assert form in (("whole",) if samples <= RULE[precision][0] else ("units", "split") if spread else ("units",))
+        assert form in (("whole",) if samples <= WHOLE_SAMPLES[precision] else ("units", "split") if spread else ("units",))
     s = scene_mod.multi_object(seed=5, w=w, h=h, n_views=9, n_src=8, f=0.8 * w)
     params = hp.default_params(radius=radius, stride=stride, top_k=top_k, precision=precision)
     with hp.Context(0) as ctx:

@@ -63,12 +63,14 @@ UNITS, ROOMY, SPLIT, WHOLE = range(4)
 
 
 def _form(f16, samples, sources, tiles, sms):
-    whole, many, few, few_max = (100, 50, 100, 2.25) if f16 else (27, 24, 100, 8)
     if 2 * tiles <= 3 * sms:
         return ROOMY
-    if samples <= whole:
+    if samples <= (100 if f16 else 27):
         return WHOLE
-    most = min(8, samples / many) if sources >= 3 else min(few_max, samples / few)
+    if f16:
+        most = 2.2 if sources < 3 else min(8, max(2.2, samples * sources / 175))
+    else:
+        most = min(8, samples / (100 if sources == 2 else 24))
     return SPLIT if 0 < 2 * (tiles % sms) <= sms and tiles <= most * sms else UNITS
 
 
