@@ -785,13 +785,17 @@ struct Dispatch {
         const PassForm form = pass_form(sc.memo ? PASS_RULE_F16 : PASS_RULE_F16_SINGLE, N, bl->max_sources,
                                         bl->total_tiles, device_sms());
         if constexpr (TH == 8) {
-            if (form == PassForm::ROOMY) return pass<R, ST, 4, PassForm::ROOMY>(*bl, sc, iteration, color, st);
-            if (form == PassForm::SPLIT) return pass<R, ST, 4, PassForm::SPLIT>(*bl, sc, iteration, color, st);
+            if (form == PassForm::ROOMY || form == PassForm::SPLIT) {  // one kernel
+                SolveConsts k = sc;
+                k.roomy = form == PassForm::ROOMY;
+                return pass<R, ST, 4, PassForm::SPLIT>(*bl, k, iteration, color, st);
+            }
         }
         // Units earn their keep by the trial bound; a half-pass on caller maps goes without it (1921 x 1081, the call,
         // units -> whole: r 7 s 2, 6 sources 3329 -> 3201 us, 1 source 692 -> 641; r 1 s 1, 6 sources 941 -> 783).
-        if (form == PassForm::WHOLE || !sc.memo)
-            return pass<R, ST, 4, PassForm::WHOLE>(*bl, sc, iteration, color, st);
+        if constexpr (TH == 8 || N <= PASS_RULE_F16.whole)
+            if (form == PassForm::WHOLE || !sc.memo)
+                return pass<R, ST, 4, PassForm::WHOLE>(*bl, sc, iteration, color, st);
         return pass<R, ST, D, PassForm::UNITS>(*bl, sc, iteration, color, st);
     }
     template <int R, int ST>

@@ -85,6 +85,7 @@ struct SolveConsts {
     int tile_h;          // rows of a CTA's tile (TILE_W x tile_h pixels, tile_h warps): 8, or 4 (FP16 path)
     int staging;         // FP16 path: quad loads in flight per window row, 4 or 8
     int memo;            // half-passes keep and use the settled bit of stored costs (whole solves: 1)
+    int roomy = 0;       // the launch leaves SMs with idle warps (PassForm::ROOMY; set by the launchers)
 };
 
 // What a launch of half-passes runs (red_black_pass), by what fills its SMs.

@@ -506,9 +506,12 @@ cudaError_t launch_rs(const BatchList& bl, const SolveConsts& sc, int iteration,
         return cudaGetLastError();
     }
     switch (pass_form(PASS_RULE_F32, N, bl.max_sources, tiles, sms)) {
-        case PassForm::ROOMY:
-            propagate_kernel<R, ST, PassForm::ROOMY><<<2 * tiles, CTA_THREADS, 0, st>>>(bl, sc, iteration, color);
+        case PassForm::ROOMY: {
+            SolveConsts k = sc;
+            k.roomy = 1;
+            propagate_kernel<R, ST, PassForm::ROOMY><<<2 * tiles, CTA_THREADS, 0, st>>>(bl, k, iteration, color);
             break;
+        }
         case PassForm::SPLIT:
             propagate_kernel<R, ST, PassForm::SPLIT><<<2 * tiles, CTA_THREADS, 0, st>>>(bl, sc, iteration, color);
             break;

@@ -201,7 +201,7 @@ __device__ __forceinline__ void red_black_pass(const ViewDesc* v, int x0, int y0
     const int kk = min(sc.top_k, S);
     // With warps idle, two parts of few sources would take two turns where one takes one.  A half-pass on caller maps
     // (memo off) scores every trial whole.
-    const int lead = !sc.memo || (K::FORM == PassForm::ROOMY && S <= 3) ? S : S - kk + 1;
+    const int lead = !sc.memo || (sc.roomy && S <= 3) ? S : S - kk + 1;
     float drange = __fmul_rn(__fsub_rn(v->dmax, v->dmin), 0.5f);
     float nrange = 1.0f;
     for (int i = 0; i < iteration; ++i) {
